@@ -195,12 +195,12 @@ __device__ __forceinline__ double broaden(int model, double eps, double x) {
   }
 }
 
-// ------------------------------------------------------- FP64 contraction
-// acc_im[p,f] = sum_t w_t reO_t(p) delta(dE_t - w_f), acc_re[p,f] = -sum_t w_t imO_t(p) delta(...)
-// over the transitions whose window covers f (src/pmx_chi.cpp:573-627) or over
-// all transitions (src/pmx_chi_copy.cpp:546-575). One CTA computes a 12x12
-// block of (a, b) = (3m+i, 3n+j) pairs for 64 frequencies; the tile's
-// transition range is contiguous because transitions are sorted by window start.
+// ---------------------------- FP64 contraction with the principal-value term
+// (epsLL and epsxyz with kk = 0): the sums of contract64.cu over all transitions
+// (src/pmx_chi_copy.cpp:546-575), and with them the principal-value sums of
+// src/pmx_chi_copy.cpp:597-615, whose weights depend on the block (i, j) of a
+// pair, so that they are not one more matrix product. One CTA computes a 12x12
+// block of (a, b) = (3m+i, 3n+j) pairs for 64 frequencies.
 namespace {
 constexpr int kMB = 4;              // m per block
 constexpr int kAB = 3 * kMB;        // a (or b) per block
@@ -219,8 +219,7 @@ __device__ __forceinline__ void tile_of(int id, int& ta, int& tb) {
   tb = id - r * (r + 1) / 2;
 }
 
-template <int NCH, bool PV>
-__global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a) {
+__global__ void __launch_bounds__(kCThreads) contract_pv_kernel(ContractArgs a) {
   int ta, tb;
   tile_of(blockIdx.x, ta, tb);
   const int f_lo = blockIdx.y * kFT;
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
   const int A = 3 * a.neps;
   const int a0 = ta * kAB, b0 = tb * kAB;
   extern __shared__ __align__(16) unsigned char smraw[];
-  typedef double2 MTile[kAB][NCH];
+  typedef double2 MTile[kAB];
   typedef double PRow[kTK + 1];
   typedef double WTile[kTK][kFT];
   MTile* sMa = reinterpret_cast<MTile*>(smraw);
@@ -236,23 +235,21 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
   PRow* sP1 = reinterpret_cast<PRow*>(sMb + kTK);
   PRow* sP2 = sP1 + kPairs;
   WTile* sW = reinterpret_cast<WTile*>(sP2 + kPairs);
-  double* sw = reinterpret_cast<double*>(sW + (PV ? 4 : 1));
+  double* sw = reinterpret_cast<double*>(sW + 4);
   double* sde = sw + kTK;
   int* sf0 = reinterpret_cast<int*>(sde + kTK);
   const int tid = threadIdx.x;
   const int pg = tid / 16, fg = tid % 16;
   double acc1[9][4], acc2[9][4];  // 1: Im (reO), 2: Re (-imO)
-  double pv1[PV ? 9 : 1][4], pv2[PV ? 9 : 1][4];
+  double pv1[9][4], pv2[9][4];
 #pragma unroll
   for (int u = 0; u < 9; ++u)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       acc1[u][q] = 0;
       acc2[u][q] = 0;
-      if (PV) {
-        pv1[u][q] = 0;
-        pv2[u][q] = 0;
-      }
+      pv1[u][q] = 0;
+      pv2[u][q] = 0;
     }
   int pclass[9];
 #pragma unroll
@@ -264,17 +261,16 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
   for (int t0 = tr.x; t0 < tr.y; t0 += kTK) {
     const int nt = min(kTK, tr.y - t0);
     // stage M of the chunk
-    for (int idx = tid; idx < kTK * kAB * NCH; idx += kCThreads) {
-      const int t = idx / (kAB * NCH), rem = idx % (kAB * NCH);
-      const int aa = rem / NCH, ch = rem % NCH;
+    for (int idx = tid; idx < kTK * kAB; idx += kCThreads) {
+      const int t = idx / kAB, aa = idx % kAB;
       double2 va = make_double2(0, 0), vb = make_double2(0, 0);
       if (t < nt) {
-        const size_t base = (size_t)(t0 + t) * A * NCH;
-        if (a0 + aa < A) va = a.M[base + (size_t)(a0 + aa) * NCH + ch];
-        if (b0 + aa < A) vb = a.M[base + (size_t)(b0 + aa) * NCH + ch];
+        const size_t base = (size_t)(t0 + t) * A;
+        if (a0 + aa < A) va = a.M[base + a0 + aa];
+        if (b0 + aa < A) vb = a.M[base + b0 + aa];
       }
-      sMa[t][aa][ch] = va;
-      sMb[t][aa][ch] = vb;
+      sMa[t][aa] = va;
+      sMb[t][aa] = vb;
     }
     if (tid < kTK) {
       const int t = tid;
@@ -287,27 +283,9 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
     for (int idx = tid; idx < kPairs * kTK; idx += kCThreads) {
       const int pp = idx / kTK, t = idx % kTK;
       const int ia = pp / kAB, ib = pp % kAB;
-      double reO, imO;
-      if (NCH == 1) {
-        const double2 o = cmulc(sMb[t][ib][0], sMa[t][ia][0]);  // a conj(b)
-        reO = o.x;
-        imO = o.y;
-      } else {
-        const double2 up_a = sMa[t][ia][0], dn_a = sMa[t][ia][1], ud_a = sMa[t][ia][2], du_a = sMa[t][ia][3];
-        const double2 up_b = sMb[t][ib][0], dn_b = sMb[t][ib][1], ud_b = sMb[t][ib][2], du_b = sMb[t][ib][3];
-        double2 tt = cmulc(up_b, up_a);
-        tt = cadd(tt, cmulc(dn_b, dn_a));
-        tt = csub(tt, cmulc(ud_b, ud_a));
-        tt = csub(tt, cmulc(du_b, du_a));
-        double2 cr = cmulc(dn_b, up_a);
-        cr = cadd(cr, cmulc(up_b, dn_a));
-        cr = csub(cr, cmulc(ud_b, du_a));
-        cr = csub(cr, cmulc(du_b, ud_a));
-        reO = tt.x + cr.x;
-        imO = tt.y;
-      }
-      sP1[pp][t] = sw[t] * reO;
-      sP2[pp][t] = -sw[t] * imO;
+      const double2 o = cmulc(sMb[t][ib], sMa[t][ia]);  // a conj(b)
+      sP1[pp][t] = sw[t] * o.x;
+      sP2[pp][t] = -sw[t] * o.y;
     }
     // weights
     for (int idx = tid; idx < kTK * kFT; idx += kCThreads) {
@@ -318,14 +296,12 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
       const double om = a.dfreq * f;
       if (in) wv = broaden(a.delta, a.eps, sde[t] - om);
       sW[0][t][fl] = wv;
-      if (PV) {
-        const double de = sde[t];
-        const double den = de * de - om * om;
-        const bool ok = t < nt && f < a.nf;
-        sW[1][t][fl] = ok ? de / den : 0.0;          // LL
-        sW[2][t][fl] = ok ? 1.0 / den : 0.0;         // LT
-        sW[3][t][fl] = ok ? 1.0 / de / den : 0.0;    // TT
-      }
+      const double de = sde[t];
+      const double den = de * de - om * om;
+      const bool ok = t < nt && f < a.nf;
+      sW[1][t][fl] = ok ? de / den : 0.0;          // LL
+      sW[2][t][fl] = ok ? 1.0 / den : 0.0;         // LT
+      sW[3][t][fl] = ok ? 1.0 / de / den : 0.0;    // TT
     }
     __syncthreads();
     for (int t = 0; t < nt; ++t) {
@@ -340,13 +316,11 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
           acc1[u][q] = fma(p1, wv[q], acc1[u][q]);
           acc2[u][q] = fma(p2, wv[q], acc2[u][q]);
         }
-        if (PV) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const double g = sW[pclass[u]][t][fg + 16 * q];
-            pv1[u][q] = fma(p1, g, pv1[u][q]);   // Re2 += w Re(O) g
-            pv2[u][q] = fma(-p2, g, pv2[u][q]);  // Im2 += w Im(O) g
-          }
+        for (int q = 0; q < 4; ++q) {
+          const double g = sW[pclass[u]][t][fg + 16 * q];
+          pv1[u][q] = fma(p1, g, pv1[u][q]);   // Re2 += w Re(O) g
+          pv2[u][q] = fma(-p2, g, pv2[u][q]);  // Im2 += w Im(O) g
         }
       }
     }
@@ -368,48 +342,27 @@ __global__ void __launch_bounds__(kCThreads) contract_f64_kernel(ContractArgs a)
       if (f >= a.nf) continue;
       a.acc[row + f] = acc2[u][q];        // Re part
       a.acc[blk + row + f] = acc1[u][q];  // Im part
-      if (PV) {
-        a.acc_pv[row + f] = pv1[u][q];
-        a.acc_pv[blk + row + f] = pv2[u][q];
-      }
+      a.acc_pv[row + f] = pv1[u][q];
+      a.acc_pv[blk + row + f] = pv2[u][q];
     }
   }
 }
 
-cudaError_t launch_contract_f64(const ContractArgs& a, cudaStream_t st) {
+cudaError_t launch_contract_pv(const ContractArgs& a, cudaStream_t st) {
   const int nmb = (a.neps + kMB - 1) / kMB;
   const int ntiles = nmb * (nmb + 1) / 2;
   const int nft = (a.nf + kFT - 1) / kFT;
   dim3 grid(ntiles, nft);
-  const bool pv = a.acc_pv != nullptr;
-  auto smem = [](int nch, bool p) {
-    return (size_t)2 * kTK * kAB * nch * sizeof(double2) + (size_t)2 * kPairs * (kTK + 1) * sizeof(double) +
-           (size_t)(p ? 4 : 1) * kTK * kFT * sizeof(double) + (size_t)2 * kTK * sizeof(double) +
-           (size_t)kTK * sizeof(int);
-  };
-  cudaError_t err;
-#define PMX_LAUNCH_CONTRACT(NCH_, PV_)                                                              \
-  {                                                                                                 \
-    const size_t sm = smem(NCH_, PV_);                                                              \
-    err = cudaFuncSetAttribute(contract_f64_kernel<NCH_, PV_>,                                       \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);               \
-    if (err != cudaSuccess) return err;                                                             \
-    contract_f64_kernel<NCH_, PV_><<<grid, kCThreads, sm, st>>>(a);                                 \
-  }
-  if (a.nch == 1) {
-    if (pv)
-      PMX_LAUNCH_CONTRACT(1, true)
-    else
-      PMX_LAUNCH_CONTRACT(1, false)
-  } else {
-    if (pv) return cudaErrorInvalidValue;
-    PMX_LAUNCH_CONTRACT(4, false)
-  }
-#undef PMX_LAUNCH_CONTRACT
+  if (a.nch != 1 || !a.acc_pv) return cudaErrorInvalidValue;
+  const size_t sm = (size_t)2 * kTK * kAB * sizeof(double2) + (size_t)2 * kPairs * (kTK + 1) * sizeof(double) +
+                    (size_t)4 * kTK * kFT * sizeof(double) + (size_t)2 * kTK * sizeof(double) +
+                    (size_t)kTK * sizeof(int);
+  const cudaError_t err =
+      cudaFuncSetAttribute(contract_pv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (err != cudaSuccess) return err;
+  contract_pv_kernel<<<grid, kCThreads, sm, st>>>(a);
   return cudaGetLastError();
 }
-
-int contract_ftile() { return kFT; }
 
 // ---------------------------------------------------------------- scaling
 // epsij: chi = SCALEFACTOR acc / w_f^2 with 1/w_0^2 := 0 (src/pmx_chi.cpp:559-563, :631-634).

@@ -46,6 +46,7 @@
 
 #include "pmx_common.cuh"
 #include "pmx_device.hpp"
+#include "pmx_dmma.cuh"
 #include "pmx_trieig.cuh"
 
 namespace pmx {
@@ -65,23 +66,6 @@ constexpr int kVecBlock = 32;  // eigenvectors per back-transform CTA
 // columns XOR-swizzled by the row so that the tensor-core fragment loads of
 // 8 rows x 4 columns and of 4 rows x 8 columns are free of bank conflicts
 __device__ __forceinline__ int pidx(int r, int c) { return r * kNB + (c ^ (r & 7)); }
-
-// D += A B for one 8x8 (A 8x4 row-major, B 4x8 column-major) FP64 MMA.
-// Fragments: a = A[lane/4][lane%4], b = B[lane%4][lane/4],
-// d0/d1 = D[lane/4][2 (lane%4) + 0/1].
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-      : "+d"(d0), "+d"(d1)
-      : "d"(a), "d"(b));
-}
-
-// acc (re/im 8x8 block) += a * b in complex arithmetic, four real MMAs
-__device__ __forceinline__ void cmma(double (&cr)[2], double (&ci)[2], double2 a, double2 b) {
-  dmma(cr[0], cr[1], a.x, b.x);
-  dmma(cr[0], cr[1], -a.y, b.y);
-  dmma(ci[0], ci[1], a.x, b.y);
-  dmma(ci[0], ci[1], a.y, b.x);
-}
 
 // acc -= a * conj(b') where the B fragment element is b'(row k, col j) taken
 // from a matrix stored as X[j][k] (so the product is V X^H)

@@ -135,7 +135,13 @@ bool overlap_tiles(int ncd_max, int nvd_max, int n, int npw, int& cchunk, int& v
 // CTA, more CTAs per SM). Every shape computes the same M. Returns the count
 // (0: no shape fits).
 int overlap_tile_candidates(int ncd_max, int nvd_max, int n, int npw, int* cc, int* vc, int maxc);
-cudaError_t launch_contract_f64(const ContractArgs& a, cudaStream_t st);
+// FP64 contraction on the FP64 tensor cores (contract64.cu); T transitions,
+// ws: contract64_workspace_bytes
+cudaError_t launch_contract64(const ContractArgs& a, long long T, double* ws, cudaStream_t st);
+size_t contract64_workspace_bytes(const ContractArgs& a, long long T);
+// FP64 contraction with the principal-value sums (acc_pv, one channel)
+cudaError_t launch_contract_pv(const ContractArgs& a, cudaStream_t st);
+// frequencies per transition range (ContractArgs::trange)
 int contract_ftile();
 cudaError_t launch_scale(const ScaleArgs& s, cudaStream_t st);
 cudaError_t launch_kk(const double* chi, double* out, int rows, int nf, double dfreq, cudaStream_t st);

@@ -268,7 +268,7 @@ struct pmx_ctx {
   // named workspaces
   DevBuf crystal, g, hkl, vloc, vso, items, hbuf, wbuf, zk, zq, scratch, info, rbuf, kgrid;
   DevBuf loci, kpts, uvec, ssoc, qgn, ncd, nvd, cbase, vbase, cidx, vidx, blkoff, dest;
-  DevBuf M, dE, wgt, f0, trange, acc, accpv, chi, chi2, mixws, epsm, stats;
+  DevBuf M, dE, wgt, f0, trange, acc, accpv, chi, chi2, c64ws, mixws, epsm, stats;
   DevBuf t_wk, t_wq, t_kw, t_ntr, t_nblk, t_toff, t_rsrc, t_rde, t_rw, t_rf0, t_cnt, t_sum;  // device transition list
   DevBuf m32, tcerr;  // tensor-core overlaps of the mixed path and their wait status
   // adjoint workspaces
@@ -954,6 +954,21 @@ const Transitions& build_transitions(const Problem& p, int soc, int nval, const 
   return T;
 }
 
+// Half width in frequency steps beyond which the line shape of epsLL and epsxyz
+// is exactly zero, or -1 where it is not within the grid (Lorentzian, broad
+// lines): a Gaussian's exp() below exp(-745.2) in FP64; in the mixed path the
+// FP32 weight, below 2^-150. Triangle and rectangle end at epsilon / 2.
+int line_support(const Problem& p, bool mixed) {
+  if (p.delta == 1 || !(p.epsilon > 0) || !std::isfinite(p.epsilon)) return -1;
+  double r = 0.5;
+  if (p.delta == 0) {
+    const double norm = 1.0 / (p.epsilon * std::sqrt(2.0 * pmx::kPi));
+    r = std::sqrt(2.0 * (mixed ? 104.0 + std::max(0.0, std::log(norm)) : 746.0));
+  }
+  const double half = std::ceil(r * p.epsilon / p.dfreq) + 1.0;
+  return half < (double)p.nfreq ? (int)half : -1;
+}
+
 int window_half(const Problem& p) {
   const double df = p.dfreq;
   const int g = std::max(1, int(6.0 * p.epsilon / df));
@@ -1037,9 +1052,13 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
                    const double2* zq, int precision, double* re, double* im, bool device_out, double* epsm) {
   cudaStream_t st = ctx->stream;
   const int mode = pl.mode, nk = pl.nk, nq = pl.nq, neps = pl.neps, nf = pl.nf, np = pl.np;
-  const int nev = pl.nev, nval = pl.nval, n = pl.n, nch = pl.nch, W = pl.W, FT = pl.FT, nft = pl.nft;
+  const int nev = pl.nev, nval = pl.nval, n = pl.n, nch = pl.nch, FT = pl.FT, nft = pl.nft;
   const size_t blkvals = pl.blkvals;
   const bool pv = pl.pv;
+  // half width of a transition's window, -1: all frequencies. epsLL and epsxyz
+  // have none of their own: the frequencies where the line shape is zero are
+  // left out (the wurtzite spectrum's Gaussians reach 26 % of its grid in FP64)
+  int W = mode == 0 ? pl.W : (pv ? -1 : line_support(p, precision == PMX_PREC_MIXED));
   pmx::dev::ScaleArgs sa = pl.sa;
   const Vec3 Q = p.lat.Q[q];
   // transition list on the device (trans.cu): occupations and counts, one
@@ -1094,9 +1113,13 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
     ctx->launches += 2;
     ctx->degenerate_cuts += tsum.cuts;
     ctx->occupation_ties += tsum.ties;
-    const bool sort = mode == 0;
-    if (sort && !pmx::dev::transitions_sortable(tsum))
-      throw CudaFail("transition energies span too many frequency steps for the device sort", PMX_ERR_LIMIT);
+    bool sort = W >= 0;
+    if (sort && !pmx::dev::transitions_sortable(tsum)) {
+      if (mode == 0)
+        throw CudaFail("transition energies span too many frequency steps for the device sort", PMX_ERR_LIMIT);
+      sort = false;
+      W = -1;
+    }
     const size_t T0 = (size_t)std::max<long long>(tsum.T, 1);
     CK(ctx->dest.ensure(sizeof(long long) * (size_t)std::max<long long>(tsum.nblk, 1)));
     CK(ctx->dE.ensure(sizeof(double) * T0));
@@ -1286,10 +1309,16 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
     ca.pvclass = mode == 2 ? 3 : 0;
     ca.wait_ns = ctx->wait_ns;
     ca.fault = ctx->fault;
-    if (precision == PMX_PREC_FP64 || pv) {
+    if (pv) {
       KTime kt(ctx, "contract_f64");
-      CK(pmx::dev::launch_contract_f64(ca, st));
+      CK(pmx::dev::launch_contract_pv(ca, st));
       ctx->launches += 1;
+    } else if (precision == PMX_PREC_FP64) {
+      const size_t wsb = pmx::dev::contract64_workspace_bytes(ca, Tn);
+      CK(ctx->c64ws.ensure(wsb));
+      KTime kt(ctx, "contract_f64");
+      CK(pmx::dev::launch_contract64(ca, Tn, ctx->c64ws.as<double>(), st));
+      ctx->launches += wsb ? 2 : 1;
     } else {
       int nl = 0;
       CK(ctx->mixws.ensure(std::max<size_t>(pmx::dev::mixed_workspace_bytes(ca, Tn), 16)));
