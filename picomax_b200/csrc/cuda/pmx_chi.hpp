@@ -144,7 +144,15 @@ cudaError_t launch_contract_pv(const ContractArgs& a, cudaStream_t st);
 // frequencies per transition range (ContractArgs::trange)
 int contract_ftile();
 cudaError_t launch_scale(const ScaleArgs& s, cudaStream_t st);
+// Kramers-Kronig transform of chi [2][rows][nf] into out: by direct sums (any nf),
+// and by FFT (kk_fft.cu, nf <= kk_fft_max_nf) with the tables of that nf in ws
+// (kk_fft_table_bytes, filled by launch_kk_tables); transposed: of the adjoint
 cudaError_t launch_kk(const double* chi, double* out, int rows, int nf, double dfreq, cudaStream_t st);
+int kk_fft_max_nf();
+size_t kk_fft_table_bytes(int nf);
+cudaError_t launch_kk_tables(int nf, void* ws, cudaStream_t st);
+cudaError_t launch_kk_fft(const double* in, double* out, int rows, int nf, double dfreq, bool transposed, void* ws,
+                          cudaStream_t st);
 
 }  // namespace dev
 }  // namespace pmx

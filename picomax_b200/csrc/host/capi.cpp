@@ -268,7 +268,7 @@ struct pmx_ctx {
   // named workspaces
   DevBuf crystal, g, hkl, vloc, vso, items, hbuf, wbuf, zk, zq, scratch, info, rbuf, kgrid;
   DevBuf loci, kpts, uvec, ssoc, qgn, ncd, nvd, cbase, vbase, cidx, vidx, blkoff, dest;
-  DevBuf M, dE, wgt, f0, trange, acc, accpv, chi, chi2, c64ws, mixws, epsm, stats;
+  DevBuf M, dE, wgt, f0, trange, acc, accpv, chi, chi2, c64ws, kktab, mixws, epsm, stats;
   DevBuf t_wk, t_wq, t_kw, t_ntr, t_nblk, t_toff, t_rsrc, t_rde, t_rw, t_rf0, t_cnt, t_sum;  // device transition list
   DevBuf m32, tcerr;  // tensor-core overlaps of the mixed path and their wait status
   // adjoint workspaces
@@ -276,6 +276,7 @@ struct pmx_ctx {
   DevBuf a_lamk, a_lamq, a_C, a_X, a_R, a_SV, a_SSO, a_kp, a_linv, a_hk, a_trik, a_triq, a_work;
   // several crystals at once (batched entry points)
   DevBuf b_g, b_hkl, b_vloc, b_vso, b_crystal;
+  int kk_nf = 0;                       // grid length of the Kramers-Kronig tables in kktab (0: none)
   double m2_err = 0.0, m2_max = 0.0;  // |M|^2 error of the mixed path's FP32 overlaps (last call)
   long long mixed_mmas = 0;            // tcgen05 MMA instructions of the mixed contractions so far
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // 0-1 stage timers, 2-3 the autotuner
@@ -354,6 +355,29 @@ int guarded(pmx_ctx* ctx, F&& f) {
     ctx->err = e.what();
     return PMX_ERR_INVALID;
   }
+}
+
+// Kramers-Kronig transform (or its transpose) of 2 rows spectra on the context's
+// stream: by FFT up to kk_fft_max_nf frequencies, whose tables are kept for the
+// grid length last used; by direct sums beyond (the transform no longer fits in
+// shared memory) and where the squared frequencies leave the FP64 range.
+void kk_transform(pmx_ctx* c, const double* in, double* out, int rows, int nf, double dfreq, bool transposed) {
+  const double step = std::abs(dfreq);
+  if (nf <= pmx::dev::kk_fft_max_nf() && step > 1e-100 && step < 1e100) {
+    if (c->kk_nf != nf) {
+      c->kk_nf = 0;
+      CK(c->kktab.ensure(pmx::dev::kk_fft_table_bytes(nf)));
+      CK(pmx::dev::launch_kk_tables(nf, c->kktab.ptr, c->stream));
+      c->kk_nf = nf;
+      c->launches += 2;
+    }
+    CK(pmx::dev::launch_kk_fft(in, out, rows, nf, dfreq, transposed, c->kktab.ptr, c->stream));
+  } else if (transposed) {
+    CK(pmx::dev::launch_kk_t(in, out, rows, nf, dfreq, c->stream));
+  } else {
+    CK(pmx::dev::launch_kk(in, out, rows, nf, dfreq, c->stream));
+  }
+  c->launches += 1;
 }
 
 void h2d(pmx_ctx* c, DevBuf& b, const void* src, size_t bytes) {
@@ -1361,8 +1385,7 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
     ctx->launches += 1;
     if (p.kk) {
       KTime kt(ctx, "kk");
-      CK(pmx::dev::launch_kk(ctx->chi.as<double>(), ctx->chi2.as<double>(), 9 * np, nf, p.dfreq, st));
-      ctx->launches += 1;
+      kk_transform(ctx, ctx->chi.as<double>(), ctx->chi2.as<double>(), 9 * np, nf, p.dfreq, false);
     }
   }
   // copy out into [i][j][q][m][n][f]
@@ -1690,8 +1713,7 @@ extern "C" int pmx_kk(pmx_ctx* ctx, int nrows, int nfreq, double dfreq, double* 
     CK(ctx->chi2.ensure(sizeof(double) * 2 * blk));
     CK(cudaMemcpyAsync(ctx->chi.ptr, re, sizeof(double) * blk, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->chi.as<double>() + blk, im, sizeof(double) * blk, cudaMemcpyHostToDevice, ctx->stream));
-    CK(pmx::dev::launch_kk(ctx->chi.as<double>(), ctx->chi2.as<double>(), nrows, nfreq, dfreq, ctx->stream));
-    ctx->launches += 1;
+    kk_transform(ctx, ctx->chi.as<double>(), ctx->chi2.as<double>(), nrows, nfreq, dfreq, false);
     CK(cudaMemcpyAsync(re, ctx->chi2.ptr, sizeof(double) * blk, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(im, ctx->chi2.as<double>() + blk, sizeof(double) * blk, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -2015,8 +2037,7 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
                          sizeof(double) * rowv, cudaMemcpyDeviceToDevice, st));
       if (p.kk) {
         KTime kt(ctx, "adj_kk");
-        CK(pmx::dev::launch_kk_t(ctx->chi2.as<double>(), ctx->a_kk.as<double>(), np, nf, p.dfreq, st));
-        ctx->launches += 1;
+        kk_transform(ctx, ctx->chi2.as<double>(), ctx->a_kk.as<double>(), np, nf, p.dfreq, true);
       } else {
         CK(cudaMemcpyAsync(ctx->a_kk.ptr, ctx->chi2.ptr, sizeof(double) * 2 * rowv, cudaMemcpyDeviceToDevice, st));
       }
