@@ -119,9 +119,9 @@ __host__ __device__ __forceinline__ long long ceil_sum(long long M) {
 __host__ __device__ __forceinline__ long long sweep_first(int ld, int s) { return ceil_sum(ld - 1) - ceil_sum(ld - 1 - s); }
 // Slot of an item in the reflector buffer (double2 offsets): the band
 // reflectors [ceil_sum(ld - 1)][16], the tridiagonal (2 ld doubles), and, in
-// launches with ld > kSmemLd, a work area of 32 ld double2: stage 1's Y
+// launches with ld > kSmemLd, a work area of 32 (ld + 16) double2: stage 1's Y
 // (16 (ld - 16)) and, for ld > kVSmemLd, V after it (16 (ld - 16)); then
-// stage 2's band (32 ld).
+// stage 2's band (32 (ld + 16)).
 __host__ __device__ __forceinline__ long long band_off(int ld) { return ceil_sum(ld - 1) * kNB + ld; }
 
 // ------------------------------------------------------------------ stage 1
@@ -549,30 +549,53 @@ __global__ void __launch_bounds__(kThr, 1) sb_kernel(const EigItem* __restrict__
 
 // ------------------------------------------------------------------ stage 2
 // Band storage Bd[c * kBandLd + d] = A(c + d, c), d = 0..31: the band and the
-// bulge (a task reaches d = len + 15 <= 31 at most). kBandLd is even, so reads
-// along a row of the band (stride kBandLd - 1) and down a column (stride 1)
-// are both free of bank conflicts.
+// bulge (a task reaches d = 31 at most), with kNB zero columns after the last
+// one: a task that sticks out of the matrix works on zeros (its reflectors are
+// zero there), so that no task checks a row or column.
 //
-// Task (s, j) (sweep s, step j, first row p = s + 1 + 16 j) reads and writes
-// exactly the elements (r, c) with p <= c < p + 16 and c <= r < p + 32 (its
-// diagonal block D and the block E below it), plus column s when j = 0. Two
-// tasks of different sweeps commute unless those sets meet, and task (s, j)
-// meets sweep s - 1 only in its steps j' <= j + 1. So sweep s may run step j
-// as soon as sweep s - 1 has finished min(j + 2, its step count) steps: each
-// pair of warps runs its sweeps s = pair, pair + 8, ... and publishes its
-// progress in a shared-memory word (release), which the next sweep's pair
-// waits for (acquire, bounded by a time limit). No block-wide barrier runs
-// between steps.
+// Task (s, j) (sweep s, step j, first row p = s + 1 + 16 j) applies reflector j
+// of the sweep two-sidedly to its diagonal block D = A(p : p+16, p : p+16) and
+// from the right to the block E = A(p+16 : p+32, p : p+16) below it; E's first
+// column then gives reflector j + 1, applied to E from the left. It touches
+// exactly the elements (r, c) with p <= c < p + 16 and c <= r < p + 32, plus
+// column s when j = 0, so it meets sweep s - 1 only in that sweep's steps <= j + 1.
+//
+// Eight pairs of warps, pair = s mod 8, a D warp and an E warp each. Both publish
+// their progress in shared-memory words (release) that other warps wait for
+// (acquire, bounded by a time limit), in half steps:
+//   D  reflector 0 formed (from column s, whose last writers are D(s-1, 0) and
+//      the first half of E(s-1, 0)): 2 j + 1 = 1; D(s, j) done: 2 (j + 1)
+//   E  E(s, j) H applied, reflector j + 1 formed: 2 j + 1; E(s, j) done: 2 (j + 1)
+// D(s, j) needs E(s-1, j) and D(s-1, j+1); E(s, j) needs those and only the first
+// half of E(s-1, j+1), of whose block it touches one element, the corner (first
+// row and column) that is final then. Within a sweep D(s, j) waits for E's
+// reflector, and E, before it writes a reflector slot, for D to have left it. No
+// barrier of any kind between steps.
+//
+// Bound by latency: a sweep follows the one before it one and a half E tasks
+// behind, so a matrix takes about 1.5 (ld - 1) E tasks, whatever the number of
+// pairs. E is therefore kept short: all offsets relative to p are fixed per lane
+// (one base address a step), sums are fused multiply-adds, a reflector takes one
+// rsqrt and one reciprocal, both halves of the warp keep the first column so that
+// its norm takes four shuffles, and the sweep's first reflector is D's work.
+// Measured on a B200: 296 matrices of n = 274 2.31 -> 1.58 ms, 148 of n = 570
+// (band in global memory) 4.84 -> 4.02 ms, against tasks that waited for whole
+// tasks of the sweep before, with a barrier per step and checks of every row and
+// column (1770 warp instructions a task, now 1000 with the polls).
 constexpr int kBandLd = 2 * kNB;
 constexpr int kPairs = 8;                // sweeps in flight: one per pair of warps
 constexpr int kS2Thr = 64 * kPairs;      // a D warp and an E warp per pair
 constexpr int kS2W = kS2Thr / 32;
-constexpr int kProgStride = 64;          // progress word: sweep * 64 + steps done (<= 26)
+constexpr int kProgStride = 128;         // progress word: sweep * 128 + half steps done
+// a reflector slot: entries 0..7 at 0, 8..15 at 9 (the two halves of a warp read
+// them from different banks), tau at 17
+constexpr int kSlot = 18;
+__device__ __forceinline__ int vidx(int r) { return r + (r >> 3); }
 constexpr long long kWaitNs = 2000000000LL;  // default limit of one wait
 
+__host__ __device__ inline size_t band_double2(int ld) { return (size_t)(ld + kNB) * kBandLd; }
 __host__ __device__ inline size_t sbtrd_smem_bytes(int ld, bool bg) {
-  return sizeof(double2) * ((bg ? 0 : (size_t)ld * kBandLd) + kPairs * 2 * 17 + kS2W * 2 * kNB) +
-         sizeof(int) * (kPairs + 4);
+  return sizeof(double2) * ((bg ? 0 : band_double2(ld)) + kPairs * 2 * kSlot + kS2W * kSlot) + sizeof(int) * (2 * kPairs + 4);
 }
 
 __device__ __forceinline__ int ld_acquire_shared(const int* p) {
@@ -593,13 +616,17 @@ __device__ __forceinline__ long long global_ns() {
   return t;
 }
 
-// Waits until *flag >= need, polling every ~kPollNs so that a waiting warp
-// leaves the issue slots to the warps that work. Gives up, and sets *err,
-// after limit_ns, after 2^28 polls, or at once when another warp has given
-// up already.
-constexpr unsigned kPollNs = 40;
+// Waits until *flag >= need: a few polls at once, then one every ~kPollNs so
+// that a waiting warp leaves the issue slots to the warps that work. Gives up,
+// and sets *err, after limit_ns, after 2^28 polls, or at once when another warp
+// has given up already.
+constexpr unsigned kPollNs = 20;
+constexpr int kSpin = 8;
 __device__ __forceinline__ void wait_progress(const int* flag, int need, int* err, long long limit_ns) {
-  if (ld_acquire_shared(flag) >= need) return;
+#pragma unroll 1
+  for (int k = 0; k < kSpin; ++k)
+    if (ld_acquire_shared(flag) >= need) return;
+  if (*reinterpret_cast<volatile int*>(err)) return;
   const long long t0 = global_ns();
   for (int k = 1; k < (1 << 28); ++k) {
     __nanosleep(kPollNs);
@@ -610,6 +637,62 @@ __device__ __forceinline__ void wait_progress(const int* flag, int need, int* er
     }
   }
   atomicExch(err, 1);
+}
+__device__ __forceinline__ void publish(int* flag, int v, int lane) {
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_block();
+    st_release_shared(flag, v);
+  }
+}
+
+// acc += a b, acc += conj(a) b, acc -= a b, acc -= a conj(b)
+__device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) {
+  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfmac(double2& acc, double2 a, double2 b) {
+  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfms(double2& acc, double2 a, double2 b) {
+  acc.x = fma(-a.x, b.x, fma(a.y, b.y, acc.x));
+  acc.y = fma(-a.x, b.y, fma(-a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfmsc(double2& acc, double2 a, double2 b) {
+  acc.x = fma(-a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
+}
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ void add_halves(double2& v) {
+  v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+  v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+}
+
+// make_refl on a short dependency chain: 1 / beta is the reciprocal square root,
+// beta its product with the sum corrected by one Newton step (to the rounding
+// of a square root)
+__device__ __forceinline__ Refl make_refl_fast(double2 alpha, double xn) {
+  Refl r;
+  if (xn == 0.0 && alpha.y == 0.0) {
+    r.tau = make_double2(0, 0);
+    r.beta = alpha.x;
+    r.scal = make_double2(1, 0);
+  } else {
+    const double s2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn));
+    const double rs = rsqrt(s2);
+    double nrm = s2 * rs;
+    nrm = fma(0.5 * rs, fma(-nrm, nrm, s2), nrm);
+    r.beta = -copysign(nrm, alpha.x);
+    const double ib = -copysign(rs, alpha.x);
+    const double2 den = make_double2(alpha.x - r.beta, alpha.y);
+    const double idd = 1.0 / fma(den.x, den.x, den.y * den.y);
+    r.tau = make_double2(fma(-alpha.x, ib, 1.0), -alpha.y * ib);
+    r.scal = make_double2(den.x * idd, -den.y * idd);
+  }
+  return r;
 }
 
 // KBG: the band in the item's work area of the reflector buffer (ld >
@@ -625,184 +708,179 @@ __global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restr
   double2* R = rbuf + it.r_off;
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* Bd = KBG ? R + band_off(ld) : reinterpret_cast<double2*>(smraw);
-  // [pair][2][17]: v (v_0 = 1), tau of the pair's next steps
-  double2* slots = KBG ? reinterpret_cast<double2*>(smraw) : Bd + (size_t)ld * kBandLd;
-  double2* wsm = slots + kPairs * 2 * 17;       // [warp][32]: [0, 16) v, [16, 32) vectors broadcast in a warp
-  int* prog = reinterpret_cast<int*>(wsm + kS2W * 2 * kNB);  // [pair]: progress words
-  int* err = prog + kPairs;                                  // a wait gave up
-  for (int idx = tid; idx < ld * kBandLd; idx += kS2Thr) {
+  // [pair][2][kSlot]: v (v_0 = 1), tau of the pair's next steps
+  double2* slots = KBG ? reinterpret_cast<double2*>(smraw) : Bd + band_double2(ld);
+  double2* wsm = slots + kPairs * 2 * kSlot;                 // [warp][kSlot]: a vector broadcast in the warp
+  int* prog_d = reinterpret_cast<int*>(wsm + kS2W * kSlot);  // [pair]: progress of the D and E warps
+  int* prog_e = prog_d + kPairs;
+  int* err = prog_e + kPairs;                                // a wait gave up
+  for (int idx = tid; idx < (ld + kNB) * kBandLd; idx += kS2Thr) {
     const int c = idx / kBandLd, d = idx % kBandLd;
     Bd[idx] = (d <= kNB && c + d < ld) ? A[(size_t)c * ld + c + d] : make_double2(0, 0);
   }
-  if (tid < kPairs) prog[tid] = -1;
+  if (tid < 2 * kPairs) prog_d[tid] = -1;
   if (tid == 0) *err = 0;
   __syncthreads();
-  // A(r, c) for 0 <= r - c <= 31 (int arithmetic, never a negative offset)
-  auto at = [&](int r, int c) -> double2& { return Bd[c * kBandLd + (r - c)]; };
   const int i = lane & 15, h = lane >> 4;
   const int pair = wid >> 1;
   const bool ewarp = (wid & 1) != 0;  // E (bulge) warp, else D (diagonal block) warp
-  double2* wv = wsm + wid * 2 * kNB;
-  double2* sl = slots + pair * 2 * 17;
+  double2* wv = wsm + wid * kSlot;
+  double2* sl = slots + pair * 2 * kSlot;
   const long long limit = it.wait_ns > 0 ? it.wait_ns : kWaitNs;
+  // offsets from Bd + p kBandLd. D element (i, 8h + cc): on or below the diagonal
+  // at column 8h + cc, above it the conjugate at column i; up: bit cc set where above
+  int doff[8];
+  unsigned up = 0;
+#pragma unroll
+  for (int cc = 0; cc < 8; ++cc) {
+    const int c = 8 * h + cc;
+    doff[cc] = c <= i ? c * (kBandLd - 1) + i : i * (kBandLd - 1) + c;
+    if (c > i) up |= 1u << cc;
+  }
+  // E element (i, 8h + cc) at e_off + cc (kBandLd - 1); (8h + rr, column i) at t_off + rr
+  const int e_off = 8 * h * (kBandLd - 1) + kNB + i;
+  const int t_off = i * (kBandLd - 1) + kNB + 8 * h;
   for (int s = pair; s <= ld - 2; s += kPairs) {
     const int ns = sweep_steps(ld, s), nprev = s > 0 ? sweep_steps(ld, s - 1) : 0;
-    const long long ridx = sweep_first(ld, s);
-    for (int j = 0; j < ns; ++j) {
-      const int p = s + 1 + kNB * j, len = min(kNB, ld - p), q = p + len;
-      if (s > 0) {  // sweep s - 1 has left the rows of this task
-        const int need = (it.wait_fault && s == 1) ? INT_MAX : (s - 1) * kProgStride + min(j + 2, nprev);
-        wait_progress(&prog[(s - 1) % kPairs], need, err, limit);
-        __syncwarp();
+    const int base = s * kProgStride, pbase = (s - 1) * kProgStride, pp = (s - 1) & (kPairs - 1);
+    // this pair's previous sweep is finished
+    const int own_done = s >= kPairs ? base - kPairs * kProgStride + 2 * sweep_steps(ld, s - kPairs) : INT_MIN;
+    const bool stuck = it.wait_fault && s == 1;
+    double2* Rs = R + sweep_first(ld, s) * kNB;
+    double2* B = Bd + (size_t)(s + 1) * kBandLd;  // column p
+    if (!ewarp) {
+      // ---- reflector 0 from column s (rows s + 1 .. s + 16), which becomes
+      // (beta, 0, ...): nothing reads it again before the tridiagonal is extracted
+      if (s > 0) {
+        wait_progress(&prog_e[pp], stuck ? INT_MAX : pbase + 1, err, limit);
+        wait_progress(&prog_d[pp], pbase + 2, err, limit);
       }
-      // this step's reflector: tau, v (all 16 entries at vsrc, v_0 = 1, zero
-      // beyond len), v_i and v at this lane's columns 8h .. 8h + 7
-      double2 tau, vi, vc[8];
-      double beta = 0.0;
-      const double2* vsrc;
-      if (j == 0) {
-        // from column s, rows p .. p + len - 1 (both warps)
-        const double2* cs = Bd + (size_t)s * kBandLd + 1;  // A(p + k, s) = cs[k]
-        // |x_1..|^2 over the 16 lanes of a half (lane i holds cs[i])
-        const double2 xi = i < len ? cs[i] : make_double2(0, 0);
-        double xx = i >= 1 ? xi.x * xi.x + xi.y * xi.y : 0.0;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) xx += __shfl_xor_sync(0xffffffffu, xx, o);
-        const Refl Rf = make_refl(cs[0], xx);
-        tau = Rf.tau;
-        beta = Rf.beta;
-        vi = i == 0 ? make_double2(1, 0) : (i < len ? cmul(xi, Rf.scal) : make_double2(0, 0));
-        if (h == 0) wv[i] = vi;
-        if (!ewarp && h == 0) R[ridx * kNB + i] = i == 0 ? tau : vi;
-        __syncwarp();
-        vsrc = wv;
-      } else {
-        vsrc = sl + (j & 1) * 17;
-        tau = vsrc[16];
-        vi = vsrc[i];
+      wait_progress(&prog_e[pair], own_done, err, limit);
+      double2* cs = B - kBandLd + 1;
+      const double2 xi = cs[i];
+      const double xx = sum16(i >= 1 ? fma(xi.x, xi.x, xi.y * xi.y) : 0.0);
+      const Refl Rf = make_refl_fast(cs[0], xx);
+      __syncwarp();
+      if (h == 0) {
+        const double2 v = i == 0 ? make_double2(1, 0) : cmul(xi, Rf.scal);
+        sl[vidx(i)] = v;
+        if (i == 0) sl[17] = Rf.tau;
+        Rs[i] = i == 0 ? Rf.tau : v;
+        cs[i] = make_double2(i == 0 ? Rf.beta : 0.0, 0.0);
       }
-#pragma unroll
-      for (int cc = 0; cc < 8; ++cc) vc[cc] = vsrc[8 * h + cc];
+      publish(&prog_d[pair], base + 1, lane);
+    }
+    for (int j = 0; j < ns; ++j, B += kNB * kBandLd) {
+      const double2* vsrc = sl + (j & 1) * kSlot;
       if (!ewarp) {
-        // ---- D <- H^H D H on D = A(p : p+len, p : p+len): lane (row i, half h)
-        double2 d[8];
+        // ---- D <- H^H D H: lane (row i, half h)
+        if (s > 0) {
+          wait_progress(&prog_e[pp], pbase + 2 * min(j + 1, nprev), err, limit);
+          wait_progress(&prog_d[pp], pbase + 2 * min(j + 2, nprev), err, limit);
+        }
+        if (j > 0) wait_progress(&prog_e[pair], base + 2 * j - 1, err, limit);
+        const double2 tau = vsrc[17], vi = vsrc[vidx(i)];
+        double2 vc[8], d[8];
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
-          const int c = 8 * h + cc;
-          // lower triangle directly, upper as the conjugate of the lower:
-          // column min(i, c), offset |i - c|
-          const int lo = c <= i ? c : i, off = c <= i ? i - c : c - i;
-          double2 val = Bd[(p + lo) * kBandLd + off];
-          if (c > i) val.y = -val.y;
-          d[cc] = (i < len && c < len) ? val : make_double2(0, 0);
+          vc[cc] = vsrc[9 * h + cc];
+          d[cc] = B[doff[cc]];
+          if (up & (1u << cc)) d[cc].y = -d[cc].y;
         }
-        double2 y0 = make_double2(0, 0), y1 = make_double2(0, 0);
+        double2 y = make_double2(0, 0), y1 = make_double2(0, 0);
 #pragma unroll
         for (int cc = 0; cc < 8; cc += 2) {
-          y0 = cadd(y0, cmul(d[cc], vc[cc]));
-          y1 = cadd(y1, cmul(d[cc + 1], vc[cc + 1]));
+          cfma(y, d[cc], vc[cc]);
+          cfma(y1, d[cc + 1], vc[cc + 1]);
         }
-        double2 y = cadd(y0, y1);
-        y.x += __shfl_xor_sync(0xffffffffu, y.x, 16);
-        y.y += __shfl_xor_sync(0xffffffffu, y.y, 16);
-        if (h == 0) wv[kNB + i] = y;
-        // v^H y = v^H D v (real; lane i holds row i's term, summed over the
-        // half's 16 lanes), w = tau y - 1/2 |tau|^2 (v^H y) v
-        double vy = vi.x * y.x + vi.y * y.y;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) vy += __shfl_xor_sync(0xffffffffu, vy, o);
+        y = cadd(y, y1);
+        add_halves(y);
+        // v^H y = v^H D v is real; w = tau y - 1/2 |tau|^2 (v^H y) v
+        const double vy = sum16(fma(vi.x, y.x, vi.y * y.y));
+        const double al = -0.5 * fma(tau.x, tau.x, tau.y * tau.y) * vy;
+        double2 w = cscale(vi, al);
+        cfma(w, tau, y);
+        if (h == 0) wv[vidx(i)] = w;
         __syncwarp();
-        const double al = -0.5 * (tau.x * tau.x + tau.y * tau.y) * vy;
-        const double2 w = cadd(cmul(tau, y), cscale(vi, al));
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
-          const int c = 8 * h + cc;
-          const double2 wc = cadd(cmul(tau, wv[kNB + c]), cscale(vc[cc], al));
-          if (i < len && c <= i) at(p + i, p + c) = csub(d[cc], cadd(cmul(vi, cconj(wc)), cmul(w, cconj(vc[cc]))));
+          cfmsc(d[cc], vi, wv[9 * h + cc]);
+          cfmsc(d[cc], w, vc[cc]);
+          if (!(up & (1u << cc))) B[doff[cc]] = d[cc];
         }
-      } else if (q < ld) {
-        // ---- E = A(q : q+len2, p : p+len) <- E H, then the next reflector
-        // from E's first column and E(:, 1:) <- H2^H E(:, 1:)
-        const int len2 = min(kNB, ld - q);
-        double2 e[8];
+        publish(&prog_d[pair], base + 2 * (j + 1), lane);
+      } else if (j + 1 < ns) {
+        // ---- E <- E H, then the next reflector from its first column and
+        // E(:, 1:) <- H2^H E(:, 1:); the sweep's last step has no E
+        if (s > 0) {
+          wait_progress(&prog_d[pp], pbase + 2 * min(j + 2, nprev), err, limit);
+          wait_progress(&prog_e[pp], stuck ? INT_MAX : pbase + min(2 * j + 3, 2 * nprev), err, limit);
+        }
+        // D has formed reflector 0; D has left the slot of reflector j + 1
+        wait_progress(&prog_d[pair], base + max(1, 2 * j), err, limit);
+        double2* Eb = B + e_off;
+        double2 vc[8], e[8];
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
-          const int c = 8 * h + cc;
-          e[cc] = (i < len2 && c < len) ? at(q + i, p + c) : make_double2(0, 0);
+          e[cc] = Eb[cc * (kBandLd - 1)];
+          vc[cc] = vsrc[9 * h + cc];
         }
-        double2 u0 = make_double2(0, 0), u1 = make_double2(0, 0);
+        const double2 tau = vsrc[17];
+        double2 u = make_double2(0, 0), u1 = make_double2(0, 0);
 #pragma unroll
         for (int cc = 0; cc < 8; cc += 2) {
-          u0 = cadd(u0, cmul(e[cc], vc[cc]));
-          u1 = cadd(u1, cmul(e[cc + 1], vc[cc + 1]));
+          cfma(u, e[cc], vc[cc]);
+          cfma(u1, e[cc + 1], vc[cc + 1]);
         }
-        double2 u = cadd(u0, u1);
-        u.x += __shfl_xor_sync(0xffffffffu, u.x, 16);
-        u.y += __shfl_xor_sync(0xffffffffu, u.y, 16);
+        u = cadd(u, u1);
+        add_halves(u);
         const double2 tu = cmul(tau, u);  // E(i, c) -= tau u_i conj(v_c)
+        cfmsc(e[0], tu, vc[0]);
+        // the first column x in both halves
+        const double2 x = shfl2(e[0], i);
+        const double xx = sum16(i >= 1 ? fma(x.x, x.x, x.y * x.y) : 0.0);
+        const Refl Rf = make_refl_fast(shfl2(x, 0), xx);
 #pragma unroll
-        for (int cc = 0; cc < 8; ++cc) e[cc] = csub(e[cc], cmul(tu, cconj(vc[cc])));
-        // E's first column x (lane (i, half 0) holds x_i) to every lane
-        if (h == 0) wv[kNB + i] = e[0];
-        // |x_1..|^2: lane (i, half 0) holds x_i = e[0] (zero for i >= len2)
-        double xx = (h == 0 && i >= 1) ? e[0].x * e[0].x + e[0].y * e[0].y : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) xx += __shfl_xor_sync(0xffffffffu, xx, o);
-        __syncwarp();
-        const Refl Rf = make_refl(wv[kNB], xx);
-        if (h == 0) e[0] = i == 0 ? make_double2(Rf.beta, 0) : make_double2(0, 0);
-#pragma unroll
-        for (int cc = 0; cc < 8; ++cc) {
-          const int c = 8 * h + cc;
-          if (i < len2 && c < len) at(q + i, p + c) = e[cc];
+        for (int cc = 1; cc < 8; ++cc) cfmsc(e[cc], tu, vc[cc]);
+        double2* nx = sl + ((j + 1) & 1) * kSlot;
+        if (h == 0) {
+          const double2 v2 = i == 0 ? make_double2(1, 0) : cmul(x, Rf.scal);
+          nx[vidx(i)] = v2;
+          if (i == 0) nx[17] = Rf.tau;
+          Rs[(j + 1) * kNB + i] = i == 0 ? Rf.tau : v2;
+          e[0] = make_double2(i == 0 ? Rf.beta : 0.0, 0.0);
         }
-        __syncwarp();
-        // E(:, 1:) <- H2^H E(:, 1:): lane (column c = i, rows of half h);
-        // v2_r = x_r scal (v2_0 = 1)
-        const double2 t2 = cconj(Rf.tau);
-        const int c = i;
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc) Eb[cc * (kBandLd - 1)] = e[cc];
+        publish(&prog_e[pair], base + 2 * j + 1, lane);
+        // lane (column i, rows 8h ..)
+        double2* Et = B + t_off;
         double2 col[8], v2r[8];
 #pragma unroll
         for (int rr = 0; rr < 8; ++rr) {
-          const int r = 8 * h + rr;
-          col[rr] = (c >= 1 && c < len && r < len2) ? at(q + r, p + c) : make_double2(0, 0);
-          v2r[rr] = r == 0 ? make_double2(1, 0) : (r < len2 ? cmul(wv[kNB + r], Rf.scal) : make_double2(0, 0));
+          col[rr] = Et[rr];
+          v2r[rr] = nx[9 * h + rr];
         }
-        double2 z0 = make_double2(0, 0), z1 = make_double2(0, 0);
+        double2 z = make_double2(0, 0), z1 = make_double2(0, 0);
 #pragma unroll
         for (int rr = 0; rr < 8; rr += 2) {
-          z0 = cadd(z0, cmulc(v2r[rr], col[rr]));
-          z1 = cadd(z1, cmulc(v2r[rr + 1], col[rr + 1]));
+          cfmac(z, v2r[rr], col[rr]);
+          cfmac(z1, v2r[rr + 1], col[rr + 1]);
         }
-        double2 zc = cadd(z0, z1);
-        zc.x += __shfl_xor_sync(0xffffffffu, zc.x, 16);
-        zc.y += __shfl_xor_sync(0xffffffffu, zc.y, 16);
-        const double2 tz = cmul(t2, zc);
+        z = cadd(z, z1);
+        add_halves(z);
+        const double2 tz = cmulc(Rf.tau, z);
+        if (i > 0) {
 #pragma unroll
-        for (int rr = 0; rr < 8; ++rr) {
-          const int r = 8 * h + rr;
-          if (c >= 1 && c < len && r < len2) at(q + r, p + c) = csub(col[rr], cmul(v2r[rr], tz));
+          for (int rr = 0; rr < 8; ++rr) {
+            cfms(col[rr], v2r[rr], tz);
+            Et[rr] = col[rr];
+          }
         }
-        if (h == 0) {
-          // the pair's next step reads the other slot buffer
-          const double2 v2 = i == 0 ? make_double2(1, 0) : (i < len2 ? cmul(wv[kNB + i], Rf.scal) : make_double2(0, 0));
-          double2* nx = sl + ((j + 1) & 1) * 17;
-          nx[i] = v2;
-          if (i == 0) nx[16] = Rf.tau;
-          R[(ridx + j + 1) * kNB + i] = i == 0 ? Rf.tau : v2;
-        }
-      }
-      // both warps of the pair are done with this step
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
-      if (!ewarp) {
-        // column s after its reflector: beta, zeros below (nothing reads it
-        // before the tridiagonal is extracted)
-        if (j == 0 && lane < len) Bd[(size_t)s * kBandLd + 1 + lane] = lane == 0 ? make_double2(beta, 0) : make_double2(0, 0);
-        __syncwarp();
-        if (lane == 0) {
-          __threadfence_block();
-          st_release_shared(&prog[pair], s * kProgStride + j + 1);
-        }
+        publish(&prog_e[pair], base + 2 * (j + 1), lane);
+      } else {
+        // both slots of the pair are free when E and D report the sweep finished
+        publish(&prog_e[pair], base + 2 * (j + 1), lane);
       }
     }
   }
@@ -1049,7 +1127,7 @@ int heev2_ld(int n) { return (n + kNB - 1) / kNB * kNB; }
 bool heev2_supported(int max_n) { return heev2_ld(max_n) >= 96 && heev2_ld(max_n) <= kMaxLd; }
 
 size_t heev2_rbuf_double2(int ld, int launch_ld) {
-  return (size_t)band_off(ld) + (launch_ld > kSmemLd ? (size_t)kBandLd * ld : 0);
+  return (size_t)band_off(ld) + (launch_ld > kSmemLd ? band_double2(ld) : 0);
 }
 
 cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nval, int max_nvec, double2* hbuf,

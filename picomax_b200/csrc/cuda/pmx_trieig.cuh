@@ -288,7 +288,7 @@ __device__ inline void tri_eigvecs(const TriWork& W, int n, int nvec, double2* _
   }
   __syncthreads();
   const int ncl = W.misc[0];
-  const double tiny = DBL_EPSILON * fmax(tnorm, DBL_MIN);
+  const double tiny = fmax(DBL_EPSILON * tnorm, 1e-290);  // its reciprocal is finite for T = 0 too
   for (int cl = tid; cl < ncl; cl += nthr) {
     double* F = scratch + cl;
     double* I0 = F + (size_t)n * ncl;
