@@ -31,9 +31,9 @@
 //  3. tri_eig_kernel: bisection and inverse iteration on the tridiagonal
 //     matrix (pmx_trieig.cuh), one CTA per matrix with small shared memory,
 //     so that many matrices share an SM.
-//  4. eig2_back_kernel: eigenvectors of T -> of the band (the bulge-chasing
-//     reflectors of one sweep act on disjoint rows: all applied at once, the
-//     sweeps in reverse) -> of H (the panels' compact WY factors in reverse).
+//  4. band_back_kernel: eigenvectors of T -> of the band (the bulge-chasing
+//     reflectors, 16 sweeps at a time, the vectors' rows in registers);
+//     panel_back_kernel: -> of H (the panels' compact WY factors in reverse).
 //
 // The matrix dimension is padded to ld = a multiple of 16 with zero rows and
 // columns: every reflector then has zero components in the padding, so T is
@@ -60,7 +60,6 @@ constexpr int kNW = kThr / 32;
 constexpr int kMaxLd = 1216;   // largest padded dimension
 constexpr int kVSmemLd = 800;  // largest one whose stage-1 V fits in shared memory
 constexpr int kSmemLd = 416;   // largest one whose stage-1 Y and stage-2 band fit in shared memory
-constexpr int kVecBlock = 32;  // eigenvectors per back-transform CTA
 
 // element (r, c) of an m x 16 complex panel in shared memory: rows of 16,
 // columns XOR-swizzled by the row so that the tensor-core fragment loads of
@@ -947,23 +946,124 @@ __global__ void __launch_bounds__(kTriThr) tri_eig_kernel(const EigItem* __restr
 }
 
 // ----------------------------------------------------------- back-transform
-constexpr int kPfSweeps = 4;  // the band reflectors are prefetched into L2 this many sweeps ahead
+// Eigenvectors of T -> of the band. The bulge-chasing reflectors (s, j) act on
+// rows s + 1 + 16 j .. + 15, and are applied with s descending; reflectors of one
+// sweep act on disjoint rows, and (s, j) meets a later sweep's reflectors only at
+// steps <= j. So the 16 sweeps of a group can be applied step by step, j
+// ascending: block (S, j) = reflectors (S + 15 .. S, j), all inside the window of
+// 32 rows from S + 16 j. One warp owns 32 / G vectors and keeps their window in
+// registers, a vector's rows r = h (mod G) in the lane (vector, h); between
+// blocks the window moves down 16 rows, so a row is read and written once per
+// group instead of once per sweep (one CTA-wide barrier per sweep before).
+// Everything is private to the warp: no barriers, vectors updated in place in
+// global memory (G neighbouring rows of a vector are one contiguous piece), the
+// next rows in registers and the next block's reflectors by cp.async meanwhile.
+// Bound by the FP64 pipe (8 FMAs per entry of a reflector and vector) with 16
+// warps per SM, by the latency of a reflector's sum and update (420 cycles) in
+// small batches. G = 4 lanes per vector: where a reflector does not start on a
+// multiple of 4, one entry more per lane meets a zero beside the staged reflector
+// (19 % of the work; 6 % with G = 2), but twice the warps of G = 2 hide more of
+// that latency and 24 vectors fill three warps: 0-4 % faster for 16 and 24 vectors
+// on 148-1184 matrices. Measured on a B200 together with panel_back_kernel against
+// one CTA per matrix with a barrier per sweep and panel columns on the CUDA cores:
+// 296 matrices of n = 274 with 17 vectors 1.25 -> 0.97 ms (1184: 4.9 -> 2.8 ms),
+// 148 of n = 570 with 25 vectors 6.1 -> 3.6 ms.
+constexpr int kBackG = 16;     // sweeps per group
+constexpr int kBackLanes = 4;  // lanes per vector
 
-__host__ __device__ inline size_t back_smem_bytes(int ld, int vb) {
-  // Z [ld][vb], one sweep's reflectors [2][ceil(ld/16)][16], W [16][vb], T [16][17]
-  return sizeof(double2) * ((size_t)ld * vb + 2 * ((ld + kNB - 1) / kNB) * kNB + kNB * vb + kNB * 17);
-}
-// reflector entries of a sweep that one thread stages (ceil(kMaxLd / 16) * 16 / 256)
-constexpr int kBackStage = (kMaxLd + kThr - 1) / kThr;
-// eigenvectors per back-transform CTA: up to kVecBlock, and few enough that
-// two CTAs share an SM (the stage is latency-bound) up to ld = 800
-inline int back_vec_block(int ld, int max_nvec) {
-  int vb = std::min(kVecBlock, std::max(max_nvec, 1));
-  // beyond ld = 800 one CTA per SM with more vectors each: every CTA reads all
-  // band reflectors (ld^2 / 2 complex) once
-  const size_t lim = (size_t)(ld > kVSmemLd ? 200 : 112) * 1024;
-  while (vb > 1 && back_smem_bytes(ld, vb) > lim) --vb;
-  return vb;
+__global__ void __launch_bounds__(32, 16) band_back_kernel(const EigItem* __restrict__ items,
+                                                      const double2* __restrict__ rbuf, double2* __restrict__ zbuf,
+                                                      const int* __restrict__ info) {
+  const EigItem it = items[blockIdx.x];
+  const int n = it.n, ld = it.ld, nvec = it.want_vec ? it.nev : 0;
+  constexpr int G = kBackLanes, kVec = 32 / G, kM = 32 / G, kHalf = kM / 2;
+  constexpr int kSt = kNB + 2 * (G - 1);  // a staged reflector with its zeros
+  const int k0 = blockIdx.y * kVec;
+  if (k0 >= nvec || info[blockIdx.x] != 0) return;
+  const int lane = threadIdx.x, h = lane % G, k = min(k0 + lane / G, nvec - 1);
+  const bool own = k0 + lane / G < nvec;  // spare lanes repeat the last vector and store nothing
+  const double2* R = rbuf + it.r_off;
+  double2* z = zbuf + it.z_off + (size_t)k * n + h;
+  __shared__ double2 sv[2 * kBackG * kSt];  // [2][16][kSt]: reflector entry q at G - 1 + q
+  __shared__ double2 st[2 * kBackG];        // [2][16]: tau
+  for (int i = lane; i < 2 * kBackG * kSt; i += 32)
+    sv[i] = make_double2(i % kSt == G - 1 ? 1.0 : 0.0, 0.0);  // v_0 = 1, zeros on both sides
+  __syncwarp();
+  // reflectors (S + t, j) into buffer b; those past the end of their sweep as zero
+  auto stage = [&](int b, int S, int j) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int t = 2 * u + (lane >> 4), q = lane & 15, s = S + t;
+      const bool ok = s <= ld - 2 && j < sweep_steps(ld, s);
+      const double2* src = R + (ok ? ((size_t)sweep_first(ld, s) + j) * kNB + q : 0);
+      double2* dst = q == 0 ? st + b * kBackG + t : sv + (b * kBackG + t) * kSt + G - 1 + q;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(ok ? 16 : 0)
+                   : "memory");
+    }
+    cp_async_commit();
+  };
+  auto load = [&](int r) { return r + h < n ? z[r] : make_double2(0, 0); };
+  for (int S = (ld - 2) / kBackG * kBackG; S >= 0; S -= kBackG) {
+    const int nj = sweep_steps(ld, S);
+    double2 w[kM];
+    stage(0, S, 0);
+#pragma unroll
+    for (int m = 0; m < kM; ++m) w[m] = load(S + G * m);
+    int p0 = S;
+    for (int j = 0; j < nj; ++j, p0 += kNB) {
+      double2 wn[kHalf];
+      if (j + 1 < nj) {
+        stage((j + 1) & 1, S, j + 1);
+#pragma unroll
+        for (int m = 0; m < kHalf; ++m) wn[m] = load(p0 + 2 * kNB + G * m);
+        cp_async_wait<1>();
+      } else {
+#pragma unroll
+        for (int m = 0; m < kHalf; ++m) wn[m] = make_double2(0, 0);
+        cp_async_wait<0>();
+      }
+      __syncwarp();
+      const double2* v = sv + (j & 1) * kBackG * kSt + h + G - 1;
+      const double2* tv = st + (j & 1) * kBackG;
+#pragma unroll
+      for (int t = kBackG - 1; t >= 0; --t) {
+        // rows t + 1 .. t + 16 of the window: entry q = G m + h - (t + 1)
+        constexpr int kE = kNB / G + 1;
+        const int m0 = (t + 1) / G, ne = (t + kNB) / G - m0 + 1;
+        double2 ve[kE], d0 = make_double2(0, 0), d1 = make_double2(0, 0);
+#pragma unroll
+        for (int e = 0; e < kE; ++e) {
+          if (e < ne) {
+            ve[e] = v[t * kSt + G * (m0 + e) - (t + 1)];
+            cfmac((e & 1) ? d1 : d0, ve[e], w[m0 + e]);
+          }
+        }
+        double2 d = cadd(d0, d1);
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          d.x += __shfl_xor_sync(0xffffffffu, d.x, o);
+          d.y += __shfl_xor_sync(0xffffffffu, d.y, o);
+        }
+        d = cmul(tv[t], d);
+#pragma unroll
+        for (int e = 0; e < kE; ++e)
+          if (e < ne) cfms(w[m0 + e], ve[e], d);
+      }
+      __syncwarp();  // the staged reflectors have been read
+#pragma unroll
+      for (int m = 0; m < kHalf; ++m) {
+        const int r = p0 + G * m;
+        if (own && r + h < n) z[r] = w[m];
+        w[m] = w[m + kHalf];
+        w[m + kHalf] = wn[m];
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kHalf; ++m) {
+      const int r = p0 + G * m;
+      if (own && r + h < n) z[r] = w[m];
+    }
+  }
 }
 
 // element r of column i of a panel's explicit V (unit diagonal, zeros above;
@@ -972,153 +1072,133 @@ __device__ __forceinline__ double2 panel_v(const double2* __restrict__ vcol, int
   return r > i ? __ldg(vcol + r) : make_double2(r == i ? 1.0 : 0.0, 0.0);
 }
 
-// Z (the eigenvectors of T, in shared memory) -> eigenvectors of H. The band
-// reflectors of a sweep are prefetched into L2 kPfSweeps sweeps earlier and
-// loaded into registers while the previous sweep is applied, then stored to
-// shared memory (one barrier per sweep); the panels' reflectors are read
-// straight from global memory (the vectors of a CTA all use the same ones,
-// so they come from L1 after the first thread).
-__global__ void __launch_bounds__(kThr, 2) eig2_back_kernel(const EigItem* __restrict__ items,
-                                                       const double2* __restrict__ hbuf,
-                                                       const double2* __restrict__ rbuf, double2* __restrict__ zbuf,
-                                                       const int* __restrict__ info, int vb) {
+// Eigenvectors of the band -> of H: the panels in reverse, Z[r0:] -= V (T (V^H
+// Z[r0:])), on the FP64 tensor cores. One CTA per matrix and 8 NB vectors, which
+// stay in shared memory; V is read straight from global memory as MMA fragments
+// (each value twice per panel, by the CTAs of a matrix from L2). Per panel: V^H Z
+// with the rows split over the warps and the partial sums added in a fixed order,
+// T times that, and the update of the rows. Two to three CTAs per SM cover the
+// three barriers and the load latency of a panel.
+template <int NB>
+__host__ __device__ constexpr int panel_ldz() { return 8 * NB + 2; }  // row stride free of bank conflicts
+template <int NB>
+inline size_t panel_back_smem(int ld) {
+  return sizeof(double2) * ((size_t)ld * panel_ldz<NB>() + 2 * kNB * panel_ldz<NB>() + kNB * 17 + (kNW / NB) * kNB * 8 * NB);
+}
+
+template <int NB>
+__global__ void __launch_bounds__(kThr, 2) panel_back_kernel(const EigItem* __restrict__ items,
+                                                           const double2* __restrict__ hbuf,
+                                                           double2* __restrict__ zbuf, const int* __restrict__ info) {
   const EigItem it = items[blockIdx.x];
   const int n = it.n, ld = it.ld, nvec = it.want_vec ? it.nev : 0;
-  const int k0 = blockIdx.y * vb;
+  constexpr int kVec = 8 * NB, kLdz = panel_ldz<NB>(), kKG = kNW / NB;
+  const int k0 = blockIdx.y * kVec;
   if (k0 >= nvec || info[blockIdx.x] != 0) return;
-  const int nv = min(vb, nvec - k0);
-  const int tid = threadIdx.x;
+  const int nv = min(kVec, nvec - k0);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, gr = lane >> 2, gk = lane & 3;
   const double2* A = hbuf + it.h_off;
-  const double2* R = rbuf + it.r_off;
-  double2* zg = zbuf + it.z_off;
+  double2* zg = zbuf + it.z_off + (size_t)k0 * n;
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int maxsteps = (ld + kNB - 1) / kNB;
-  double2* Z = reinterpret_cast<double2*>(smraw);  // Z[r * nv + k]
-  double2* RB = Z + (size_t)ld * nv;               // [2][maxsteps * 16]
-  double2* W = RB + 2 * maxsteps * kNB;            // [16][nv]
-  double2* T = W + kNB * nv;                       // [16][17]
-  for (int idx = tid; idx < ld * nv; idx += kThr) {
-    const int r = idx / nv, k = idx % nv;
-    Z[idx] = r < n ? zg[(size_t)(k0 + k) * n + r] : make_double2(0, 0);
+  double2* Z = reinterpret_cast<double2*>(smraw);  // [ld][kLdz]
+  double2* W = Z + (size_t)ld * kLdz;              // [16][kLdz] V^H Z
+  double2* W2 = W + kNB * kLdz;                    // [16][kLdz] T V^H Z
+  double2* T = W2 + kNB * kLdz;                    // [16][17]
+  double2* red = T + kNB * 17;                     // [kKG][16][kVec] partial sums
+  for (int idx = tid; idx < ld * kVec; idx += kThr) {
+    const int k = idx / ld, r = idx % ld;
+    Z[r * kLdz + k] = k < nv && r < n ? zg[(size_t)k * n + r] : make_double2(0, 0);
   }
-  auto prefetch_sweep = [&](int s) {  // one 128-byte line per thread
-    const int lines = sweep_steps(ld, s) * kNB * (int)sizeof(double2) / 128;
-    if (tid < lines)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(R + sweep_first(ld, s) * kNB + tid * (128 / sizeof(double2))));
-  };
-  for (int s = ld - 2; s > ld - 2 - kPfSweeps && s >= 0; --s) prefetch_sweep(s);
-  auto load_sweep = [&](int s, double2 (&st)[kBackStage]) {
-    const int cnt = sweep_steps(ld, s) * kNB;
-    const double2* src = R + sweep_first(ld, s) * kNB;
-#pragma unroll
-    for (int u = 0; u < kBackStage; ++u) {
-      const int idx = tid + u * kThr;
-      st[u] = idx < cnt ? __ldg(src + idx) : make_double2(0, 0);
-    }
-  };
-  auto store_sweep = [&](double2* dst, const double2 (&st)[kBackStage]) {
-#pragma unroll
-    for (int u = 0; u < kBackStage; ++u)
-      if (tid + u * kThr < maxsteps * kNB) dst[tid + u * kThr] = st[u];
-  };
-  {
-    double2 st[kBackStage];
-    load_sweep(ld - 2, st);
-    store_sweep(RB, st);
-  }
-  __syncthreads();
-  // ---- band reflectors, sweeps in reverse; one sweep's reflectors act on
-  // disjoint rows and are applied together (one thread per reflector and vector)
-  for (int s = ld - 2; s >= 0; --s) {
-    if (s - kPfSweeps >= 0) prefetch_sweep(s - kPfSweeps);
-    double2 st[kBackStage];
-    if (s > 0) load_sweep(s - 1, st);  // lands while this sweep is applied
-    const int ns = sweep_steps(ld, s);
-    const double2* Rs = RB + ((ld - 2 - s) & 1) * maxsteps * kNB;
-    for (int task = tid; task < ns * nv; task += kThr) {
-      const int j = task / nv, k = task % nv;
-      const int p = s + 1 + kNB * j, len = min(kNB, ld - p);
-      const double2* v = Rs + j * kNB;
-      const double2 tau = v[0];
-      if (tau.x == 0.0 && tau.y == 0.0) continue;
-      double2* zc = Z + (size_t)p * nv + k;
-      double2 zr[kNB];
-#pragma unroll
-      for (int q = 0; q < kNB; ++q) zr[q] = q < len ? zc[(size_t)q * nv] : make_double2(0, 0);
-      double2 d0 = zr[0], d1 = make_double2(0, 0);
-#pragma unroll
-      for (int q = 1; q < kNB; q += 2) {
-        d1 = cadd(d1, cmulc(v[q], zr[q]));
-        if (q + 1 < kNB) d0 = cadd(d0, cmulc(v[q + 1], zr[q + 1]));
-      }
-      const double2 dot = cmul(tau, cadd(d0, d1));
-      zc[0] = csub(zr[0], dot);
-#pragma unroll
-      for (int q = 1; q < kNB; ++q)
-        if (q < len) zc[(size_t)q * nv] = csub(zr[q], cmul(v[q], dot));
-    }
-    if (s > 0) store_sweep(RB + ((ld - 1 - s) & 1) * maxsteps * kNB, st);
-    __syncthreads();
-  }
-  // ---- panels in reverse: Z[r0:] -= V (T (V^H Z[r0:]))
+  const int nb = wid % NB, kg = wid / NB;  // this warp's vectors and share of the rows in V^H Z
   for (int c0 = ld - 2 * kNB; c0 >= 0; c0 -= kNB) {
     const int r0 = c0 + kNB, m = ld - r0;
-    for (int idx = tid; idx < kNB * kNB; idx += kThr) {
-      const int i = idx % kNB, j = idx / kNB;
+    const double2* Vp = A + (size_t)c0 * ld + r0;  // column i at Vp + i ld
+    if (tid < kNB * kNB) {
+      const int i = tid % kNB, j = tid / kNB;
       T[i * 17 + j] = __ldg(A + (size_t)(r0 + j) * ld + c0 + i);
     }
-    // W = V^H Z[r0:]: thread (i, k), two chains over the rows
-#pragma unroll
-    for (int o = 0; o < 2; ++o) {
-      const int idx = tid + o * kThr;
-      if (idx < kNB * nv) {
-        const int i = idx / nv, k = idx % nv;
-        const double2* vcol = A + (size_t)(c0 + i) * ld + r0;
-        const double2* zc = Z + (size_t)r0 * nv + k;
-        double2 a0 = make_double2(0, 0), a1 = make_double2(0, 0);
-        int r = i;  // V is zero above its diagonal
+    __syncthreads();  // Z of the last panel (or the load), T
+    {
+      double cr[2][2] = {{0, 0}, {0, 0}}, ci[2][2] = {{0, 0}, {0, 0}};
+      const double2* va = Vp + (size_t)gr * ld;
+      const double2* vb = va + (size_t)8 * ld;
+      const double2* zb = Z + (size_t)r0 * kLdz + 8 * nb + gr;
 #pragma unroll 4
-        for (; r + 1 < m; r += 2) {
-          a0 = cadd(a0, cmulc(panel_v(vcol, r, i), zc[(size_t)r * nv]));
-          a1 = cadd(a1, cmulc(panel_v(vcol, r + 1, i), zc[(size_t)(r + 1) * nv]));
-        }
-        if (r < m) a0 = cadd(a0, cmulc(panel_v(vcol, r, i), zc[(size_t)r * nv]));
-        W[idx] = cadd(a0, a1);
+      for (int ks = kg; ks < m / 4; ks += kKG) {
+        const int r = 4 * ks + gk;
+        const double2 a0 = cconj(ks < 4 ? panel_v(va, r, gr) : __ldg(va + r));
+        const double2 a1 = cconj(ks < 4 ? panel_v(vb, r, gr + 8) : __ldg(vb + r));
+        const double2 b = zb[r * kLdz];
+        cmma(cr[0], ci[0], a0, b);
+        cmma(cr[1], ci[1], a1, b);
       }
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+          red[((kg * kNB) + 8 * x + gr) * kVec + 8 * nb + 2 * gk + y] = make_double2(cr[x][y], ci[x][y]);
     }
     __syncthreads();
-    // W <- T W (T upper triangular): thread per column k
-    for (int k = tid; k < nv; k += kThr) {
-      double2 w[kNB];
+    for (int idx = tid; idx < kNB * kVec; idx += kThr) {
+      const int i = idx / kVec, k = idx % kVec;
+      double2 s = red[i * kVec + k];
 #pragma unroll
-      for (int i = 0; i < kNB; ++i) w[i] = W[i * nv + k];
-#pragma unroll
-      for (int i = 0; i < kNB; ++i) {
-        double2 sacc = make_double2(0, 0);
-#pragma unroll
-        for (int q = i; q < kNB; ++q) sacc = cadd(sacc, cmul(T[i * 17 + q], w[q]));
-        W[i * nv + k] = sacc;
-      }
+      for (int g = 1; g < kKG; ++g) s = cadd(s, red[(g * kNB + i) * kVec + k]);
+      W[i * kLdz + k] = s;
     }
     __syncthreads();
-    // Z[r0:] -= V W: thread (row, k)
-    for (int idx = tid; idx < m * nv; idx += kThr) {
-      const int r = idx / nv, k = idx % nv;
-      double2 s0 = make_double2(0, 0), s1 = make_double2(0, 0);
-#pragma unroll
-      for (int i = 0; i < kNB; i += 2) {
-        s0 = cadd(s0, cmul(panel_v(A + (size_t)(c0 + i) * ld + r0, r, i), W[i * nv + k]));
-        s1 = cadd(s1, cmul(panel_v(A + (size_t)(c0 + i + 1) * ld + r0, r, i + 1), W[(i + 1) * nv + k]));
-      }
-      double2* z = Z + (size_t)(r0 + r) * nv + k;
-      *z = csub(*z, cadd(s0, s1));
+    for (int idx = tid; idx < kNB * kVec; idx += kThr) {  // T upper triangular
+      const int i = idx / kVec, k = idx % kVec;
+      double2 s = make_double2(0, 0);
+      for (int q = i; q < kNB; ++q) cfma(s, T[i * 17 + q], W[q * kLdz + k]);
+      W2[i * kLdz + k] = s;
     }
     __syncthreads();
+    double2 bw[4][NB];
+#pragma unroll
+    for (int kb = 0; kb < 4; ++kb)
+#pragma unroll
+      for (int x = 0; x < NB; ++x) {
+        const double2 t = W2[(4 * kb + gk) * kLdz + 8 * x + gr];
+        bw[kb][x] = make_double2(-t.x, -t.y);
+      }
+#pragma unroll 2
+    for (int I = wid; I < m / 8; I += kNW) {
+      const int r = 8 * I + gr;
+      double2 a[4];
+#pragma unroll
+      for (int kb = 0; kb < 4; ++kb) {
+        const double2* vc = Vp + (size_t)(4 * kb + gk) * ld;
+        a[kb] = I < 2 ? panel_v(vc, r, 4 * kb + gk) : __ldg(vc + r);
+      }
+#pragma unroll
+      for (int x = 0; x < NB; ++x) {
+        double2* zp = Z + (size_t)(r0 + r) * kLdz + 8 * x + 2 * gk;
+        const double2 z0 = zp[0], z1 = zp[1];
+        double cr[2] = {z0.x, z1.x}, ci[2] = {z0.y, z1.y};
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb) cmma(cr, ci, a[kb], bw[kb][x]);
+        zp[0] = make_double2(cr[0], ci[0]);
+        zp[1] = make_double2(cr[1], ci[1]);
+      }
+    }
   }
-  for (int idx = tid; idx < n * nv; idx += kThr) {
+  __syncthreads();
+  for (int idx = tid; idx < nv * n; idx += kThr) {
     const int k = idx / n, r = idx % n;
-    zg[(size_t)(k0 + k) * n + r] = Z[(size_t)r * nv + k];
+    zg[(size_t)k * n + r] = Z[r * kLdz + k];
   }
+}
+
+template <int NB>
+cudaError_t launch_panel_back(const EigItem* items, int nitems, int ld, int max_nvec, const double2* hbuf,
+                              double2* zbuf, const int* info, cudaStream_t st) {
+  const size_t sm = panel_back_smem<NB>(ld);
+  const cudaError_t e =
+      cudaFuncSetAttribute(panel_back_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  panel_back_kernel<NB><<<dim3(nitems, (max_nvec + 8 * NB - 1) / (8 * NB)), kThr, sm, st>>>(items, hbuf, zbuf, info);
+  return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------- host
@@ -1158,14 +1238,16 @@ cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nv
   e = cudaFuncSetAttribute(tri_eig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
   if (e != cudaSuccess) return e;
   tri_eig_kernel<<<nitems, kTriThr, s3, st>>>(items, rbuf, wbuf, zbuf, scratch, info, xsm_ok);
-  if (max_nvec > 0) {
-    const int vb = back_vec_block(ld, max_nvec);
-    const size_t s4 = back_smem_bytes(ld, vb);
-    e = cudaFuncSetAttribute(eig2_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s4);
-    if (e != cudaSuccess) return e;
-    eig2_back_kernel<<<dim3(nitems, (max_nvec + vb - 1) / vb), kThr, s4, st>>>(items, hbuf, rbuf, zbuf, info, vb);
+  e = cudaGetLastError();
+  if (max_nvec > 0 && e == cudaSuccess) {
+    constexpr int kVec = 32 / kBackLanes;
+    band_back_kernel<<<dim3(nitems, (max_nvec + kVec - 1) / kVec), 32, 0, st>>>(items, rbuf, zbuf, info);
+    // 16 vectors a CTA while two CTAs share an SM (ld <= 304), else 8
+    e = max_nvec > 8 && panel_back_smem<2>(ld) <= 112 * 1024
+            ? launch_panel_back<2>(items, nitems, ld, max_nvec, hbuf, zbuf, info, st)
+            : launch_panel_back<1>(items, nitems, ld, max_nvec, hbuf, zbuf, info, st);
   }
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace dev
