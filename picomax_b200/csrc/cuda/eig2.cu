@@ -28,9 +28,9 @@
 //     sweep waiting only for the previous sweep to leave its rows (progress
 //     words in shared memory, no block-wide barrier). Reflectors go to
 //     global memory.
-//  3. tri_eig_kernel: bisection and inverse iteration on the tridiagonal
-//     matrix (pmx_trieig.cuh), one CTA per matrix with small shared memory,
-//     so that many matrices share an SM.
+//  3. tri_val_kernel, tri_vec_kernel: bisection and inverse iteration on the
+//     tridiagonal matrix (pmx_trieig.cuh), one CTA per matrix, so that many
+//     matrices share an SM.
 //  4. band_back_kernel: eigenvectors of T -> of the band (the bulge-chasing
 //     reflectors, 16 sweeps at a time, the vectors' rows in registers);
 //     panel_back_kernel: -> of H (the panels' compact WY factors in reverse).
@@ -894,28 +894,43 @@ __global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restr
 }
 
 // --------------------------------------------------------- tridiagonal stage
-// 256 threads per matrix (one CTA): multisection bisection probes 256 / nval
-// points per eigenvalue at once; the inverse iteration runs one thread per
-// eigenvalue cluster (128-thread CTAs measured slower: 1.29 vs 1.16 ms)
-constexpr int kTriThr = 256;
+// Bisection (pmx_trieig.cuh) with 256 threads per matrix, 256 / nval probes per
+// eigenvalue and round: bound by the FP64 pipe with two or more CTAs per SM, by the
+// row-to-row chain of the Sturm sequence (8 cycles) below. The eigenvectors are a
+// kernel of their own, because one thread per vector works there, for which 256
+// threads and their registers would leave the SM empty: 64 threads a matrix, with
+// the factors and iterates in global memory (in shared memory, one CTA per SM: the
+// same up to 148 matrices, 3-5 % slower solver beyond). Measured on a B200 against
+// one kernel with divisions in the Sturm chain, one thread per eigenvalue cluster
+// and four factor arrays: 296 matrices of n = 274 with 17 vectors 0.67 -> 0.12 +
+// 0.22 ms, 148 of n = 570 with 25 vectors 2.37 -> 0.16 + 0.42 ms.
+constexpr int kTriThr = 256, kTriVecThr = 64;
 
-__host__ __device__ inline size_t tri_smem_bytes(int n, int nval, int nvec) {
-  return sizeof(double) * ((size_t)3 * n + 8 + 3 * nval + kTriThr) + sizeof(int) * ((size_t)kTriThr + nvec + 1 + 4);
+inline size_t tri_smem_bytes(int n, int nval) {
+  return sizeof(double) * ((size_t)3 * n + 8 + 3 * nval + kTriThr) + sizeof(int) * (kTriThr + 4);
 }
-// with the inverse-iteration iterates in shared memory (n * nvec doubles after
-// the work arrays), when three CTAs still share an SM
-__host__ __device__ inline size_t tri_smem_xbytes(int n, int nval, int nvec) {
-  return (tri_smem_bytes(n, nval, nvec) + 7) / 8 * 8 + sizeof(double) * (size_t)n * nvec;
+inline size_t tri_vec_smem_bytes(int n, int nvec) {
+  return sizeof(double) * ((size_t)2 * n + 8 + 2 * nvec) + sizeof(int) * ((size_t)nvec + 8);
 }
-constexpr size_t kTriXsmMax = 72 * 1024;
 
-__global__ void __launch_bounds__(kTriThr) tri_eig_kernel(const EigItem* __restrict__ items,
+// T of an item: d [n] and e [n] into shared memory; false when the bulge chase
+// gave up a wait (T is incomplete)
+__device__ __forceinline__ bool load_tri(const EigItem& it, const double2* rbuf, double* d, double* e) {
+  const int n = it.n, ld = it.ld;
+  const double* de = reinterpret_cast<const double*>(rbuf + it.r_off + ceil_sum(ld - 1) * kNB);
+  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+    d[c] = de[c];
+    e[c] = c + 1 < n ? de[ld + c] : 0.0;
+  }
+  __syncthreads();
+  return de[2 * ld - 1] == 0.0;
+}
+
+__global__ void __launch_bounds__(kTriThr) tri_val_kernel(const EigItem* __restrict__ items,
                                                      const double2* __restrict__ rbuf, double* __restrict__ wbuf,
-                                                     double2* __restrict__ zbuf, double* __restrict__ scratch,
-                                                     int* __restrict__ info, int xsm_ok) {
+                                                     int* __restrict__ info) {
   const EigItem it = items[blockIdx.x];
-  const int n = it.n, ld = it.ld, nval = it.nval, nvec = it.want_vec ? it.nev : 0;
-  const int tid = threadIdx.x;
+  const int n = it.n, nval = it.nval;
   extern __shared__ __align__(16) unsigned char smraw[];
   double* d = reinterpret_cast<double*>(smraw);
   double* e = d + n;
@@ -926,23 +941,47 @@ __global__ void __launch_bounds__(kTriThr) tri_eig_kernel(const EigItem* __restr
   double* hi = lo + nval;
   double* xs = hi + nval;
   int* cnt = reinterpret_cast<int*>(xs + kTriThr);
-  int* clus = cnt + kTriThr;
-  int* misc = clus + nvec + 1;
-  const double* de = reinterpret_cast<const double*>(rbuf + it.r_off + ceil_sum(ld - 1) * kNB);
-  for (int c = tid; c < n; c += kTriThr) {
-    d[c] = de[c];
-    e[c] = c + 1 < n ? de[ld + c] : 0.0;
-  }
-  __syncthreads();
-  if (de[2 * ld - 1] != 0.0) {  // the bulge chase gave up a wait: T is incomplete
-    if (tid == 0) info[blockIdx.x] = 3;
+  if (!load_tri(it, rbuf, d, e)) {
+    if (threadIdx.x == 0) info[blockIdx.x] = 3;
     return;
   }
-  const TriWork tw{d, e, e2, red, lam, lo, hi, xs, cnt, clus, misc};
+  const TriWork tw{d, e, e2, red, lam, lo, hi, xs, cnt, nullptr, nullptr};
   const int status = tri_eigvals(tw, n, nval, wbuf + it.w_off, it.bisect_cap);
-  double* xsm = xsm_ok ? reinterpret_cast<double*>(smraw + (tri_smem_bytes(n, nval, nvec) + 7) / 8 * 8) : nullptr;
-  if (nvec > 0 && status == 0) tri_eigvecs(tw, n, nvec, zbuf + it.z_off, scratch + it.s_off, blockIdx.x, xsm);
-  if (tid == 0) info[blockIdx.x] = status;
+  if (threadIdx.x == 0) info[blockIdx.x] = status;
+}
+
+__global__ void __launch_bounds__(kTriVecThr) tri_vec_kernel(const EigItem* __restrict__ items,
+                                                        const double2* __restrict__ rbuf,
+                                                        const double* __restrict__ wbuf, double2* __restrict__ zbuf,
+                                                        double* __restrict__ scratch, const int* __restrict__ info) {
+  const EigItem it = items[blockIdx.x];
+  const int n = it.n, nvec = it.want_vec ? it.nev : 0, tid = threadIdx.x;
+  if (nvec <= 0 || info[blockIdx.x] != 0) return;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double* d = reinterpret_cast<double*>(smraw);
+  double* e = d + n;
+  double* red = e + n;
+  double* lam = red + 8;
+  double* rn = lam + nvec;
+  int* clus = reinterpret_cast<int*>(rn + nvec);
+  int* misc = clus + nvec + 1;
+  load_tri(it, rbuf, d, e);
+  // as tri_eigvals leaves T: its norm, negligible off-diagonals zero
+  double tn = 0.0;
+  for (int i = tid; i < n; i += kTriVecThr)
+    tn = fmax(tn, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
+  if ((tid & 31) == 0) red[tid >> 5] = tn;
+  __syncthreads();
+  tn = fmax(red[0], red[1]);
+  for (int i = tid; i < n - 1; i += kTriVecThr)
+    if (fabs(e[i]) <= DBL_EPSILON * (fabs(d[i]) + fabs(d[i + 1]))) e[i] = 0.0;
+  for (int k = tid; k < nvec; k += kTriVecThr) lam[k] = wbuf[it.w_off + k];
+  if (tid == 0) red[3] = tn;
+  __syncthreads();
+  const TriWork tw{d, e, nullptr, red, lam, rn, nullptr, nullptr, nullptr, clus, misc};
+  tri_eigvecs(tw, n, nvec, zbuf + it.z_off, scratch + it.s_off, blockIdx.x);
 }
 
 // ----------------------------------------------------------- back-transform
@@ -1233,11 +1272,16 @@ cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nv
   e = cudaFuncSetAttribute(tr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
   if (e != cudaSuccess) return e;
   tr<<<nitems, kS2Thr, s2, st>>>(items, hbuf, rbuf);
-  const int xsm_ok = tri_smem_xbytes(max_n, max_nval, max_nvec) <= kTriXsmMax ? 1 : 0;
-  const size_t s3 = xsm_ok ? tri_smem_xbytes(max_n, max_nval, max_nvec) : tri_smem_bytes(max_n, max_nval, max_nvec);
-  e = cudaFuncSetAttribute(tri_eig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
+  const size_t s3 = tri_smem_bytes(max_n, max_nval);
+  e = cudaFuncSetAttribute(tri_val_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
   if (e != cudaSuccess) return e;
-  tri_eig_kernel<<<nitems, kTriThr, s3, st>>>(items, rbuf, wbuf, zbuf, scratch, info, xsm_ok);
+  tri_val_kernel<<<nitems, kTriThr, s3, st>>>(items, rbuf, wbuf, info);
+  if (max_nvec > 0) {
+    const size_t s5 = tri_vec_smem_bytes(max_n, max_nvec);
+    e = cudaFuncSetAttribute(tri_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s5);
+    if (e != cudaSuccess) return e;
+    tri_vec_kernel<<<nitems, kTriVecThr, s5, st>>>(items, rbuf, wbuf, zbuf, scratch, info);
+  }
   e = cudaGetLastError();
   if (max_nvec > 0 && e == cudaSuccess) {
     constexpr int kVec = 32 / kBackLanes;
