@@ -273,7 +273,7 @@ struct pmx_ctx {
   DevBuf m32, tcerr;  // tensor-core overlaps of the mixed path and their wait status
   // adjoint workspaces
   DevBuf a_chi, a_g, a_gx, a_kk, a_f1, a_f2, a_obar, a_debar, a_mbar, a_zbk, a_zbq, a_lbk, a_lbq;
-  DevBuf a_lamk, a_lamq, a_C, a_X, a_R, a_SV, a_SSO, a_kp, a_linv, a_hk, a_trik, a_triq, a_work;
+  DevBuf a_lamk, a_lamq, a_C, a_X, a_R, a_SV, a_SSO, a_kp, a_linv, a_tri, a_work;
   // several crystals at once (batched entry points)
   DevBuf b_g, b_hkl, b_vloc, b_vso, b_crystal;
   int kk_nf = 0;                       // grid length of the Kramers-Kronig tables in kktab (0: none)
@@ -470,26 +470,45 @@ cudaError_t eig_launch(pmx_ctx* c, const pmx::dev::EigItem* items, int nitems, i
 
 // H workspace of one chunk of eigensolves: 2 GB, or up to 8 GB where two
 // waves of 148 matrices of the largest size need more (n > 832), so that the
-// large sizes still fill the GPU; 2 GB with the tridiagonal export, whose
-// callers keep their k-points within one chunk of that size
+// large sizes still fill the GPU; 4 GB and one matrix more with the tridiagonal
+// export, whose caller keeps 2 GB at k and k + q each and the reference point
+// within one chunk
 size_t h_budget(size_t hbytes_max, bool tri) {
   const size_t base = (size_t)2 << 30;
-  return tri ? base : std::max(base, std::min((size_t)8 << 30, 296 * hbytes_max));
+  return tri ? 2 * base + hbytes_max : std::max(base, std::min((size_t)8 << 30, 296 * hbytes_max));
 }
 
-// Assembles and diagonalises H(k) for every k; the lowest nval eigenvalues
-// go to w (host, [nk][nval]); with zdev the lowest nvec eigenvectors go to
-// zdev ([nk][nvec][n]).
-// With tri (device, [nk][4 n]) the tridiagonal form of every H(k) is exported
-// and the reflectors of the last chunk stay in c->hbuf (ks must then fit one
-// chunk: nk <= 2 GB / (16 n^2)).
-void solve_k(pmx_ctx* c, const DevCrystal& dc, const std::vector<Vec3>& ks, int nval, int nvec, double2* zdev,
-             std::vector<double>& w, double* tri = nullptr) {
-  const int nk = (int)ks.size(), n = dc.n;
-  w.assign((size_t)nk * nval, 0.0);
+// One set of eigenproblems of a crystal: H(k) of every k, the lowest nval
+// eigenvalues into w (host, [nk][nval]), the lowest nvec eigenvectors (0: none)
+// at z_off of the solve's vector buffer ([nk][nvec][n]).
+struct SolveSet {
+  std::vector<Vec3> ks;
+  int nval, nvec;
+  long long z_off;
+  std::vector<double>* w;
+};
+
+// Assembles and diagonalises H(k) of all sets in common launches: the solver's
+// stages take one or two matrices per SM, so that a set of its own (above all the
+// single matrix of the reference energy) would pay for a wave of SMs it does not
+// fill. zdev may be null when no set has vectors.
+// With tri (device, [items][4 n], items in set order) the tridiagonal form of every
+// H(k) is exported and the reflectors of the last chunk stay in c->hbuf (all sets
+// must then fit one chunk, see h_budget).
+void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& sets, double2* zdev,
+                double* tri = nullptr) {
+  const int n = dc.n;
+  int nk = 0, nval = 0, nvec = 0;
+  for (const SolveSet& s : sets) {
+    s.w->assign(s.ks.size() * (size_t)s.nval, 0.0);
+    if (s.ks.empty()) continue;
+    if (s.nval > n) throw CudaFail("too many eigenvalues requested", PMX_ERR_INVALID);
+    nk += (int)s.ks.size();
+    nval = std::max(nval, s.nval);
+    if (zdev) nvec = std::max(nvec, s.nvec);
+  }
   if (nk == 0) return;
-  if (nval > n) throw CudaFail("too many eigenvalues requested", PMX_ERR_INVALID);
-  const bool vec = zdev != nullptr && nvec > 0;
+  const bool vec = nvec > 0;
   const bool tri_req = tri != nullptr;
   const int ld = eig_ld(n, n, tri_req);
   const size_t hbytes = (size_t)ld * ld * sizeof(double2);
@@ -501,28 +520,35 @@ void solve_k(pmx_ctx* c, const DevCrystal& dc, const std::vector<Vec3>& ks, int 
   }
   CK(c->hbuf.ensure(hbytes * chunk));
   CK(c->wbuf.ensure(sizeof(double) * (size_t)nk * nval));
-  const size_t sstride = pmx::dev::heev_scratch_doubles(n, vec ? nvec : 0, n);
+  const size_t sstride = pmx::dev::heev_scratch_doubles(n, nvec, n);
   const bool per_item = vec || n > 832;  // without vectors the scratch holds only the large-n partial sums
   CK(c->scratch.ensure(sizeof(double) * sstride * (per_item ? chunk : 1)));
   CK(c->info.ensure(sizeof(int) * chunk));
   const size_t rstride = eig_rstride(n, n, tri_req);
   if (rstride) CK(c->rbuf.ensure(sizeof(double2) * rstride * chunk));
+  // (set, index in it) of every item
+  std::vector<std::pair<int, int>> where;
+  where.reserve(nk);
+  for (size_t s = 0; s < sets.size(); ++s)
+    for (size_t i = 0; i < sets[s].ks.size(); ++i) where.emplace_back((int)s, (int)i);
   std::vector<pmx::dev::EigItem> items(chunk);
   std::vector<int> info(chunk);
   for (int k0 = 0; k0 < nk; k0 += chunk) {
     const int cnt = std::min(chunk, nk - k0);
     for (int i = 0; i < cnt; ++i) {
       pmx::dev::EigItem& it = items[i];
+      const SolveSet& set = sets[where[k0 + i].first];
+      const int ik = where[k0 + i].second;
       it = pmx::dev::EigItem{};
       it.crystal = 0;
       it.n = n;
-      it.nev = vec ? nvec : 0;
-      it.nval = nval;
-      it.want_vec = vec ? 1 : 0;
-      for (int x = 0; x < 3; ++x) it.k[x] = ks[k0 + i][x];
+      it.nev = vec ? set.nvec : 0;
+      it.nval = set.nval;
+      it.want_vec = it.nev > 0 ? 1 : 0;
+      for (int x = 0; x < 3; ++x) it.k[x] = set.ks[ik][x];
       it.h_off = (long long)i * ld * ld;
       it.w_off = (long long)(k0 + i) * nval;
-      it.z_off = (long long)(k0 + i) * nvec * n;
+      it.z_off = set.z_off + (long long)ik * set.nvec * n;
       it.s_off = per_item ? (long long)(i * sstride) : 0;
       it.ld = ld;
       it.r_off = (long long)(i * rstride);
@@ -578,12 +604,17 @@ void solve_k(pmx_ctx* c, const DevCrystal& dc, const std::vector<Vec3>& ks, int 
     for (int i = 0; i < cnt; ++i)
       if (info[i] != 0)
         throw CudaFail("eigensolver failed (status " + std::to_string(info[i]) + ") at k-point " +
-                           std::to_string(k0 + i),
+                           std::to_string(where[k0 + i].second),
                        eig_status_error(info[i]));
   }
+  std::vector<double> w((size_t)nk * nval);
   CK(cudaMemcpyAsync(w.data(), c->wbuf.ptr, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->d2h += sizeof(double) * w.size();
+  for (int i = 0; i < nk; ++i) {
+    const SolveSet& set = sets[where[i].first];
+    std::copy_n(w.begin() + (size_t)i * nval, set.nval, set.w->begin() + (size_t)where[i].second * set.nval);
+  }
 }
 
 // Spinor eigenvalue s of a solved item (spatial spectrum doubled without SOC).
@@ -594,19 +625,27 @@ inline double spinor_eig(const std::vector<double>& w, int nev, int k, int s, in
 // Number of solved states needed to cover `spinor` spinor states.
 inline int solved_states(int spinor, int soc) { return soc ? spinor : (spinor + 1) / 2; }
 
-double ref_energy(pmx_ctx* c, const pmx_problem* P, const DevCrystal& dc) {
-  const Problem& p = P->p;
-  const int nh = 2 * p.npw();
-  if (!(p.nvalence > 0 && p.nvalence < nh)) {
-    std::cout << "WARNING::setRefEnergy:: nvalence is out of bounds for eigenvalues. Setting offset to 0."
-              << std::endl;
-    return 0.0;
-  }
-  const int nev = solved_states(p.nvalence + 1, dc.soc);
+// The eigenproblem of the reference energy (setRefEnergy, src/pmx_epm.cpp:393-428)
+// as a set of a solve, empty when nvalence is out of bounds, and the energy from
+// its eigenvalues.
+struct RefSolve {
+  int nev = 0;
   std::vector<double> w;
-  solve_k(c, dc, {p.refpoint}, nev, 0, nullptr, w);
-  return (spinor_eig(w, nev, 0, p.nvalence - 1, dc.soc) + spinor_eig(w, nev, 0, p.nvalence, dc.soc)) / 2.0;
-}
+  SolveSet set(const Problem& p, int soc, int nvec = 0, long long z_off = 0) {
+    const int nh = 2 * p.npw();
+    if (!(p.nvalence > 0 && p.nvalence < nh)) {
+      std::cout << "WARNING::setRefEnergy:: nvalence is out of bounds for eigenvalues. Setting offset to 0."
+                << std::endl;
+      return {{}, 0, 0, 0, &w};
+    }
+    nev = solved_states(p.nvalence + 1, soc);
+    return {{p.refpoint}, nev, nvec, z_off, &w};
+  }
+  double energy(const Problem& p, int soc) const {
+    if (nev == 0) return 0.0;
+    return (spinor_eig(w, nev, 0, p.nvalence - 1, soc) + spinor_eig(w, nev, 0, p.nvalence, soc)) / 2.0;
+  }
+};
 
 }  // namespace
 
@@ -744,7 +783,9 @@ extern "C" int pmx_ref_energy(pmx_ctx* ctx, const pmx_problem* P, double* off) {
   if (!P || !off) return PMX_ERR_INVALID;
   return guarded(ctx, [&]() {
     DevCrystal dc = upload_crystal(ctx, P, 0);
-    *off = ref_energy(ctx, P, dc);
+    RefSolve ref;
+    solve_sets(ctx, dc, {ref.set(P->p, dc.soc)}, nullptr);
+    *off = ref.energy(P->p, dc.soc);
     return (int)PMX_OK;
   });
 }
@@ -756,7 +797,8 @@ extern "C" int pmx_band(pmx_ctx* ctx, const pmx_problem* P, double* eband) {
     for (double& t : ctx->stage_ms) t = 0;
     Timer tm(ctx, 0);
     DevCrystal dc = upload_crystal(ctx, P, 0);
-    const double off = ref_energy(ctx, P, dc);
+    RefSolve ref;
+    const SolveSet ref_set = ref.set(p, dc.soc);
     const int nh = 2 * p.npw();
     const int nkeep = std::min(p.nband, nh);
     if (nkeep <= 0) {
@@ -765,7 +807,8 @@ extern "C" int pmx_band(pmx_ctx* ctx, const pmx_problem* P, double* eband) {
     }
     const int nev = solved_states(nkeep, dc.soc);
     std::vector<double> w;
-    solve_k(ctx, dc, p.lat.Q, nev, 0, nullptr, w);
+    solve_sets(ctx, dc, {ref_set, {p.lat.Q, nev, 0, 0, &w}}, nullptr);
+    const double off = ref.energy(p, dc.soc);
     for (int q = 0; q < p.nq(); ++q)
       for (int n = 0; n < p.nband; ++n)
         eband[(size_t)q * p.nband + n] = n < nh ? spinor_eig(w, nev, q, n, dc.soc) - off : 0.0;
@@ -1425,37 +1468,50 @@ static int run_chi(pmx_ctx* ctx, const pmx_problem* P, int sw, int precision, do
     // re/im may both be NULL when eps_M is requested (eps_M only, no chi copy-out)
     if ((!re || !im) && !(epsm && !re && !im)) return (int)PMX_ERR_INVALID;
     DevCrystal dc;
-    double off;
-    std::vector<double> wk;
+    RefSolve ref;
+    SolveSet ref_set;
     {
       Timer tm(ctx, 0);
       dc = upload_crystal(ctx, P, sw == PMX_SWITCH_EPSXYZ ? 1 : 0);
-      off = ref_energy(ctx, P, dc);
+      ref_set = ref.set(p, dc.soc);
     }
     const ChiPlan pl = chi_plan(p, sw, dc);
     const int nk = pl.nk, nev = pl.nev, nval = pl.nval, n = pl.n;
     ctx->degenerate_cuts = 0;
     ctx->occupation_ties = 0;
     ctx->m2_err = ctx->m2_max = 0.0;
-    CK(ctx->zk.ensure(std::max<size_t>(sizeof(double2) * (size_t)nk * nev * n, 16)));
-    CK(ctx->zq.ensure(std::max<size_t>(sizeof(double2) * (size_t)nk * nev * n, 16)));
-    {
-      Timer tm(ctx, 0);
-      solve_k(ctx, dc, p.K, nval, nev, ctx->zk.as<double2>(), wk);
-    }
+    // eigenvectors at k, then at k + q of a group of q's: as many q's as make about
+    // eight waves of 148 matrices with the k points, within 4 GB
+    const long long zq = (long long)nk * nev * n;
+    const long long zfit = ((long long)4 << 30) / std::max<long long>(1, zq * (long long)sizeof(double2));
+    const int group = (int)std::max<long long>(
+        1, std::min<long long>({(long long)pl.nq, (8 * 148 + nk - 1) / std::max(1, nk), zfit}));
+    CK(ctx->zk.ensure(std::max<size_t>(sizeof(double2) * (size_t)(1 + group) * zq, 16)));
     chi_tables(ctx, p);
     chi_buffers(ctx, pl);
-    for (int q = 0; q < pl.nq; ++q) {
-      const Vec3 Q = p.lat.Q[q];
-      std::vector<Vec3> kq(nk);
-      for (int k = 0; k < nk; ++k) kq[k] = p.K[k] + Q;
-      std::vector<double> wq;
+    std::vector<double> wk;
+    double off = 0.0;
+    for (int q0 = 0; q0 < pl.nq || q0 == 0; q0 += group) {
+      const int cnt = std::min(group, pl.nq - q0);
+      std::vector<std::vector<double>> wq(std::max(cnt, 0));
       {
         Timer tm(ctx, 0);
-        solve_k(ctx, dc, kq, nval, nev, ctx->zq.as<double2>(), wq);
+        std::vector<SolveSet> sets;
+        if (q0 == 0) {
+          sets.push_back(ref_set);
+          sets.push_back({p.K, nval, nev, 0, &wk});
+        }
+        for (int i = 0; i < cnt; ++i) {
+          std::vector<Vec3> kq(nk);
+          for (int k = 0; k < nk; ++k) kq[k] = p.K[k] + p.lat.Q[q0 + i];
+          sets.push_back({std::move(kq), nval, nev, (1 + i) * zq, &wq[i]});
+        }
+        solve_sets(ctx, dc, sets, ctx->zk.as<double2>());
+        if (q0 == 0) off = ref.energy(p, dc.soc);
       }
-      chi_process_q(ctx, p, pl, dc, q, off, wk, wq, ctx->zk.as<double2>(), ctx->zq.as<double2>(), precision, re,
-                    im, device_out, epsm);
+      for (int i = 0; i < cnt; ++i)
+        chi_process_q(ctx, p, pl, dc, q0 + i, off, wk, wq[i], ctx->zk.as<double2>(),
+                      ctx->zk.as<double2>() + (1 + i) * zq, precision, re, im, device_out, epsm);
     }
     CK(cudaStreamSynchronize(st));
     if (ctx->degenerate_cuts > 0)
@@ -1883,20 +1939,16 @@ void hf_items(pmx_ctx* c, const DevCrystal& dc, const double2* Z, long long zs, 
   hgrad_items(c, dc, c->a_X.as<double2>(), (long long)ns * dc.n, Z, zs, ks, ns);
 }
 
-// Gradient of the reference energy (E_{nv-1} + E_nv)/2 scaled by obar.
-void ref_energy_grad(pmx_ctx* c, const pmx_problem* P, const DevCrystal& dc, double obar) {
+// Gradient of the reference energy (E_{nv-1} + E_nv)/2 scaled by obar, from the
+// ns = solved_states(nvalence + 1) eigenvectors at the reference point.
+void ref_energy_grad(pmx_ctx* c, const pmx_problem* P, const DevCrystal& dc, const double2* z, double obar) {
   const Problem& p = P->p;
-  const int nh = 2 * p.npw();
-  if (!(p.nvalence > 0 && p.nvalence < nh) || obar == 0.0) return;
   const int ns = solved_states(p.nvalence + 1, dc.soc);
-  std::vector<double> w;
-  CK(c->zk.ensure(sizeof(double2) * (size_t)ns * dc.n));
-  solve_k(c, dc, {p.refpoint}, ns, ns, c->zk.as<double2>(), w);
   std::vector<double> lb(ns, 0.0);
   const int s1 = dc.soc ? p.nvalence - 1 : (p.nvalence - 1) / 2, s2 = dc.soc ? p.nvalence : p.nvalence / 2;
   lb[s1] += 0.5 * obar;
   lb[s2] += 0.5 * obar;
-  hf_items(c, dc, c->zk.as<double2>(), (long long)ns * dc.n, lb, {p.refpoint}, ns);
+  hf_items(c, dc, z, (long long)ns * dc.n, lb, {p.refpoint}, ns);
 }
 
 }  // namespace
@@ -1937,23 +1989,28 @@ extern "C" int pmx_band_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* dE
     if (nkeep > 0 && nq > 0) {
       const int ns = solved_states(nkeep, dc.soc), n = dc.n;
       const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nq, ((size_t)1 << 30) / ((size_t)ns * n * 16)));
-      CK(ctx->zq.ensure(sizeof(double2) * (size_t)chunk * ns * n));
+      // the reference point is solved with the first chunk, unless its gradient is zero
+      for (int q = 0; q < nq; ++q)
+        for (int s = 0; s < nkeep; ++s) osum += dE[(size_t)q * p.nband + s];
+      const bool with_ref = p.nvalence > 0 && p.nvalence < nh && osum != 0.0;
+      const int rs = with_ref ? solved_states(p.nvalence + 1, dc.soc) : 0;
+      const long long zref = (long long)chunk * ns * n;
+      CK(ctx->zq.ensure(sizeof(double2) * ((size_t)zref + (size_t)rs * n)));
       for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int cnt = std::min(chunk, nq - q0);
         std::vector<Vec3> ks(p.lat.Q.begin() + q0, p.lat.Q.begin() + q0 + cnt);
-        std::vector<double> w;
-        solve_k(ctx, dc, ks, ns, ns, ctx->zq.as<double2>(), w);
+        std::vector<double> w, wref;
+        std::vector<SolveSet> sets{{ks, ns, ns, 0, &w}};
+        if (q0 == 0 && with_ref) sets.push_back({{p.refpoint}, rs, rs, zref, &wref});
+        solve_sets(ctx, dc, sets, ctx->zq.as<double2>());
         std::vector<double> lb((size_t)cnt * ns, 0.0);
         for (int q = 0; q < cnt; ++q)
-          for (int s = 0; s < nkeep; ++s) {
-            const double g = dE[(size_t)(q0 + q) * p.nband + s];
-            lb[(size_t)q * ns + (dc.soc ? s : s / 2)] += g;
-            osum += g;
-          }
+          for (int s = 0; s < nkeep; ++s)
+            lb[(size_t)q * ns + (dc.soc ? s : s / 2)] += dE[(size_t)(q0 + q) * p.nband + s];
         hf_items(ctx, dc, ctx->zq.as<double2>(), (long long)ns * n, lb, ks, ns);
       }
+      if (with_ref) ref_energy_grad(ctx, P, dc, ctx->zq.as<double2>() + zref, -osum);
     }
-    ref_energy_grad(ctx, P, dc, -osum);
     adj_finish(ctx, P, dc, grad);
     return (int)PMX_OK;
   });
@@ -1997,11 +2054,13 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
     }
     ctx->launches += 1;
     DevCrystal dc;
-    double off;
+    RefSolve ref;
+    SolveSet ref_set;
+    double off = 0.0;
     {
       Timer tm(ctx, 0);
       dc = upload_crystal(ctx, P, has_soc_params(P) ? 1 : 0);
-      off = ref_energy(ctx, P, dc);
+      ref_set = ref.set(p, dc.soc);
     }
     adj_begin(ctx, P, dc);
     const int n = dc.n, nall = n, npw = dc.npw;
@@ -2021,7 +2080,9 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
     // degeneracy) and the reduction H = Q T Q^H of each H(k) for the resolvent
     // of the rest; a block's reflectors must fit one eigensolver chunk.
     int nsx = std::min(n, ns + 8);
-    const int kb = (int)std::max<size_t>(1, std::min<size_t>((size_t)nk, ((size_t)2 << 30) / ((size_t)n * n * 16)));
+    // (2 kb + 1 matrices make one eigensolver chunk, at most 4096)
+    const int kb = (int)std::max<size_t>(
+        1, std::min<size_t>({(size_t)nk, ((size_t)2 << 30) / ((size_t)n * n * 16), (size_t)2047}));
     (void)nall;
     CK(ctx->a_kk.ensure(sizeof(double) * 2 * (size_t)np * nf));
     CK(ctx->chi2.ensure(sizeof(double) * 2 * (size_t)np * nf));
@@ -2063,17 +2124,18 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
         for (;;) {
           nvs = nsx;
           nvl = std::min(n, nsx + 1);
-          CK(ctx->zk.ensure(sizeof(double2) * (size_t)cnt * nvs * n));
-          CK(ctx->zq.ensure(sizeof(double2) * (size_t)cnt * nvs * n));
-          CK(ctx->a_trik.ensure(sizeof(double) * 4 * (size_t)cnt * n));
-          CK(ctx->a_triq.ensure(sizeof(double) * 4 * (size_t)cnt * n));
+          // k and k + q (and once the reference point) in one solve: eigenvectors,
+          // tridiagonals and reflectors of the k side first, then of the k + q side
+          const long long zs = (long long)cnt * nvs * n;
+          CK(ctx->zk.ensure(sizeof(double2) * 2 * (size_t)zs));
+          CK(ctx->a_tri.ensure(sizeof(double) * 4 * (size_t)(2 * cnt + 1) * n));
           {
             Timer tm(ctx, 0);
-            solve_k(ctx, dc, ks, nvl, nvs, ctx->zk.as<double2>(), wk, ctx->a_trik.as<double>());
-            // keep the reflectors of the k side while the k+q side is reduced
-            std::swap(ctx->hbuf.ptr, ctx->a_hk.ptr);
-            std::swap(ctx->hbuf.bytes, ctx->a_hk.bytes);
-            solve_k(ctx, dc, kqs, nvl, nvs, ctx->zq.as<double2>(), wq, ctx->a_triq.as<double>());
+            std::vector<SolveSet> sets{{ks, nvl, nvs, 0, &wk}, {kqs, nvl, nvs, zs, &wq}};
+            const bool first = ref.w.empty() && !ref_set.ks.empty();
+            if (first) sets.push_back(ref_set);
+            solve_sets(ctx, dc, sets, ctx->zk.as<double2>(), ctx->a_tri.as<double>());
+            if (first) off = ref.energy(p, dc.soc);
           }
           // the projected prefix must not split a degenerate set
           bool split = false;
@@ -2128,7 +2190,7 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
             if (!pmx::dev::overlap_tiles(ncd_max, nvd_max, n, npw, oa.cchunk, oa.vchunk))
               throw CudaFail("overlap tile does not fit in shared memory", PMX_ERR_UNSUPPORTED);
             oa.zk = ctx->zk.as<double2>();
-            oa.zq = ctx->zq.as<double2>();
+            oa.zq = (ctx->zk.as<double2>() + (long long)cnt * nvs * n);
             oa.ncd = ctx->ncd.as<int>();
             oa.nvd = ctx->nvd.as<int>();
             oa.cbase = ctx->cbase.as<int>();
@@ -2199,7 +2261,7 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
           za.ncd_max = ncd_max;
           za.nvd_max = nvd_max;
           za.zk = ctx->zk.as<double2>();
-          za.zq = ctx->zq.as<double2>();
+          za.zq = (ctx->zk.as<double2>() + (long long)cnt * nvs * n);
           za.ncd = ctx->ncd.as<int>();
           za.nvd = ctx->nvd.as<int>();
           za.cbase = ctx->cbase.as<int>();
@@ -2231,7 +2293,7 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
         CK(ctx->a_X.ensure(sizeof(double2) * (size_t)cnt * ns * n));
         CK(ctx->a_work.ensure(sizeof(double) * (size_t)cnt * 8 * 5 * n));
         for (int side = 0; side < 2; ++side) {
-          const double2* Z = side == 0 ? ctx->zk.as<double2>() : ctx->zq.as<double2>();
+          const double2* Z = side == 0 ? ctx->zk.as<double2>() : (ctx->zk.as<double2>() + (long long)cnt * nvs * n);
           const double2* Zb = side == 0 ? ctx->a_zbk.as<double2>() : ctx->a_zbq.as<double2>();
           const double* lam = side == 0 ? ctx->a_lamk.as<double>() : ctx->a_lamq.as<double>();
           const double* lb = side == 0 ? ctx->a_lbk.as<double>() : ctx->a_lbq.as<double>();
@@ -2254,8 +2316,8 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
             ra.ns = ns;
             ra.nsx = nsx;
             ra.nitems = cnt;
-            ra.H = side == 0 ? ctx->a_hk.as<double2>() : ctx->hbuf.as<double2>();
-            ra.tri = side == 0 ? ctx->a_trik.as<double>() : ctx->a_triq.as<double>();
+            ra.H = ctx->hbuf.as<double2>() + (side == 0 ? 0 : (size_t)cnt * n * n);
+            ra.tri = ctx->a_tri.as<double>() + (side == 0 ? 0 : (size_t)4 * cnt * n);
             ra.lam = lam;
             ra.lam_stride = nvl;
             ra.Z = Z;
@@ -2524,33 +2586,17 @@ void solve_multi(pmx_ctx* c, const pmx::dev::CrystalDev* table, std::vector<Solv
   }
 }
 
-// Reference energies of every problem in one merged solve (setRefEnergy,
-// src/pmx_epm.cpp:393-428).
-std::vector<double> ref_energies(pmx_ctx* c, const pmx_problem* const* P, int count, const DevCrystalSet& set) {
-  std::vector<double> off(count, 0.0);
-  std::vector<std::vector<double>> w(count);
-  std::vector<SolveReq> reqs;
+// Appends the reference point of every problem to a merged solve.
+void ref_requests(const pmx_problem* const* P, int count, const DevCrystalSet& set, std::vector<RefSolve>& ref,
+                  std::vector<SolveReq>& reqs) {
+  ref.assign(count, RefSolve{});
   for (int i = 0; i < count; ++i) {
-    const Problem& p = P[i]->p;
-    const int nh = 2 * p.npw();
-    if (!(p.nvalence > 0 && p.nvalence < nh)) {
-      std::cout << "WARNING::setRefEnergy:: nvalence is out of bounds for eigenvalues. Setting offset to 0."
-                << std::endl;
-      continue;
-    }
     const DevCrystal& d = set.dc[i];
-    const int nev = solved_states(p.nvalence + 1, d.soc);
-    w[i].assign(nev, 0.0);
-    reqs.push_back({i, d.n, d.npw, p.refpoint, nev, 0, 0, w[i].data()});
+    const SolveSet s = ref[i].set(P[i]->p, d.soc);
+    if (s.ks.empty()) continue;
+    ref[i].w.assign(s.nval, 0.0);
+    reqs.push_back({i, d.n, d.npw, s.ks[0], s.nval, 0, 0, ref[i].w.data()});
   }
-  solve_multi(c, set.table, reqs, nullptr);
-  for (int i = 0; i < count; ++i) {
-    if (w[i].empty()) continue;
-    const Problem& p = P[i]->p;
-    const int soc = set.dc[i].soc, nev = (int)w[i].size();
-    off[i] = (spinor_eig(w[i], nev, 0, p.nvalence - 1, soc) + spinor_eig(w[i], nev, 0, p.nvalence, soc)) / 2.0;
-  }
-  return off;
 }
 
 }  // namespace
@@ -2563,9 +2609,10 @@ extern "C" int pmx_band_batch(pmx_ctx* ctx, int count, const pmx_problem* const*
     for (double& t : ctx->stage_ms) t = 0;
     Timer tm(ctx, 0);
     const DevCrystalSet set = upload_crystals(ctx, problems, count);
-    const std::vector<double> off = ref_energies(ctx, problems, count, set);
+    std::vector<RefSolve> ref;
     std::vector<std::vector<double>> w(count);
     std::vector<SolveReq> reqs;
+    ref_requests(problems, count, set, ref, reqs);
     for (int i = 0; i < count; ++i) {
       const Problem& p = problems[i]->p;
       const DevCrystal& d = set.dc[i];
@@ -2585,9 +2632,10 @@ extern "C" int pmx_band_batch(pmx_ctx* ctx, int count, const pmx_problem* const*
         continue;
       }
       const int nev = solved_states(nkeep, set.dc[i].soc);
+      const double off = ref[i].energy(p, set.dc[i].soc);
       for (int q = 0; q < p.nq(); ++q)
         for (int b = 0; b < p.nband; ++b)
-          eband[i][(size_t)q * p.nband + b] = b < nh ? spinor_eig(w[i], nev, q, b, set.dc[i].soc) - off[i] : 0.0;
+          eband[i][(size_t)q * p.nband + b] = b < nh ? spinor_eig(w[i], nev, q, b, set.dc[i].soc) - off : 0.0;
     }
     return (int)PMX_OK;
   });
@@ -2612,11 +2660,12 @@ extern "C" int pmx_chi_batch(pmx_ctx* ctx, int count, const pmx_problem* const* 
     ctx->occupation_ties = 0;
     ctx->m2_err = ctx->m2_max = 0.0;
     DevCrystalSet set;
-    std::vector<double> off;
+    std::vector<RefSolve> ref;
+    std::vector<SolveReq> ref_reqs;  // solved with the first group's k points
     {
       Timer tm(ctx, 0);
       set = upload_crystals(ctx, problems, count, sw == PMX_SWITCH_EPSXYZ ? 1 : 0);
-      off = ref_energies(ctx, problems, count, set);
+      ref_requests(problems, count, set, ref, ref_reqs);
     }
     std::vector<ChiPlan> pl;
     for (int i = 0; i < count; ++i) pl.push_back(chi_plan(problems[i]->p, sw, set.dc[i]));
@@ -2635,50 +2684,44 @@ extern "C" int pmx_chi_batch(pmx_ctx* ctx, int count, const pmx_problem* const* 
       std::vector<long long> zo(g1 - g0 + 1, 0);
       for (int i = g0; i < g1; ++i)
         zo[i - g0 + 1] = zo[i - g0] + (long long)pl[i].nk * pl[i].nev * pl[i].n;
-      CK(ctx->zk.ensure(std::max<size_t>(sizeof(double2) * (size_t)zo.back(), 16)));
-      CK(ctx->zq.ensure(std::max<size_t>(sizeof(double2) * (size_t)zo.back(), 16)));
-      // k stage of every problem of the group
+      // eigenvectors at k, then at k + q
+      CK(ctx->zk.ensure(std::max<size_t>(sizeof(double2) * 2 * (size_t)zo.back(), 16)));
       std::vector<std::vector<double>> wk(count);
-      {
-        Timer tm(ctx, 0);
-        std::vector<SolveReq> reqs;
-        for (int i = g0; i < g1; ++i) {
-          const Problem& p = problems[i]->p;
-          const DevCrystal& d = set.dc[i];
-          wk[i].assign((size_t)pl[i].nk * pl[i].nval, 0.0);
-          for (int k = 0; k < pl[i].nk; ++k)
-            reqs.push_back({i, d.n, d.npw, p.K[k], pl[i].nval, pl[i].nev,
-                            zo[i - g0] + (long long)k * pl[i].nev * pl[i].n, wk[i].data() + (size_t)k * pl[i].nval});
-        }
-        solve_multi(ctx, set.table, reqs, ctx->zk.as<double2>());
-      }
       int maxq = 0;
       for (int i = g0; i < g1; ++i) maxq = std::max(maxq, pl[i].nq);
-      for (int q = 0; q < maxq; ++q) {
-        // k+q stage of every problem that has this q, then each problem's chi
+      for (int q = 0; q < std::max(maxq, 1); ++q) {
+        // k + q stage of every problem that has this q, with the k stage and (in the
+        // first group) the reference points when q = 0, then each problem's chi
         std::vector<std::vector<double>> wq(count);
         {
           Timer tm(ctx, 0);
           std::vector<SolveReq> reqs;
+          if (q == 0) reqs.swap(ref_reqs);
           for (int i = g0; i < g1; ++i) {
-            if (q >= pl[i].nq) continue;
             const Problem& p = problems[i]->p;
             const DevCrystal& d = set.dc[i];
+            const long long zs = (long long)pl[i].nev * pl[i].n;
+            if (q == 0) {
+              wk[i].assign((size_t)pl[i].nk * pl[i].nval, 0.0);
+              for (int k = 0; k < pl[i].nk; ++k)
+                reqs.push_back({i, d.n, d.npw, p.K[k], pl[i].nval, pl[i].nev, zo[i - g0] + k * zs,
+                                wk[i].data() + (size_t)k * pl[i].nval});
+            }
+            if (q >= pl[i].nq) continue;
             wq[i].assign((size_t)pl[i].nk * pl[i].nval, 0.0);
             for (int k = 0; k < pl[i].nk; ++k)
               reqs.push_back({i, d.n, d.npw, p.K[k] + p.lat.Q[q], pl[i].nval, pl[i].nev,
-                              zo[i - g0] + (long long)k * pl[i].nev * pl[i].n,
-                              wq[i].data() + (size_t)k * pl[i].nval});
+                              zo.back() + zo[i - g0] + k * zs, wq[i].data() + (size_t)k * pl[i].nval});
           }
-          solve_multi(ctx, set.table, reqs, ctx->zq.as<double2>());
+          solve_multi(ctx, set.table, reqs, ctx->zk.as<double2>());
         }
         for (int i = g0; i < g1; ++i) {
           if (q >= pl[i].nq) continue;
           const Problem& p = problems[i]->p;
           chi_tables(ctx, p);
           chi_buffers(ctx, pl[i]);
-          chi_process_q(ctx, p, pl[i], set.dc[i], q, off[i], wk[i], wq[i], ctx->zk.as<double2>() + zo[i - g0],
-                        ctx->zq.as<double2>() + zo[i - g0], precision, re ? re[i] : nullptr,
+          chi_process_q(ctx, p, pl[i], set.dc[i], q, ref[i].energy(p, set.dc[i].soc), wk[i], wq[i],
+                        ctx->zk.as<double2>() + zo[i - g0], ctx->zk.as<double2>() + zo.back() + zo[i - g0], precision, re ? re[i] : nullptr,
                         im ? im[i] : nullptr, false, epsm ? epsm[i] : nullptr);
         }
       }
