@@ -75,6 +75,24 @@ __device__ __forceinline__ void cmma_sub_herm(double (&cr)[2], double (&ci)[2], 
   dmma(ci[0], ci[1], -a.y, x.x);
 }
 
+// acc += a b, acc += conj(a) b, acc -= a b, acc -= a conj(b)
+__device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) {
+  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfmac(double2& acc, double2 a, double2 b) {
+  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfms(double2& acc, double2 a, double2 b) {
+  acc.x = fma(-a.x, b.x, fma(a.y, b.y, acc.x));
+  acc.y = fma(-a.x, b.y, fma(-a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfmsc(double2& acc, double2 a, double2 b) {
+  acc.x = fma(-a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
+}
+
 // sum over the first `w` lanes' groups: xor reductions within 16 lanes
 __device__ __forceinline__ double sum16(double v) {
 #pragma unroll
@@ -90,6 +108,10 @@ struct Refl {
   double beta;
   double2 scal;
 };
+// 1 / beta is the reciprocal square root, beta its product with the sum corrected
+// by one Newton step (to the rounding of a square root): one rsqrt and one
+// reciprocal, where a square root and two divisions took twice the instructions
+// on the chain that every column and every bulge waits for.
 __device__ __forceinline__ Refl make_refl(double2 alpha, double xn) {
   Refl r;
   if (xn == 0.0 && alpha.y == 0.0) {
@@ -97,11 +119,15 @@ __device__ __forceinline__ Refl make_refl(double2 alpha, double xn) {
     r.beta = alpha.x;
     r.scal = make_double2(1, 0);
   } else {
-    // two independent divisions: 1 / beta and 1 / |alpha - beta|^2
-    r.beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn), alpha.x);
+    const double s2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn));
+    const double rs = rsqrt(s2);
+    double nrm = s2 * rs;
+    nrm = fma(0.5 * rs, fma(-nrm, nrm, s2), nrm);
+    r.beta = -copysign(nrm, alpha.x);
+    const double ib = -copysign(rs, alpha.x);
     const double2 den = make_double2(alpha.x - r.beta, alpha.y);
-    const double ib = 1.0 / r.beta, idd = 1.0 / (den.x * den.x + den.y * den.y);
-    r.tau = make_double2(1.0 - alpha.x * ib, -alpha.y * ib);
+    const double idd = 1.0 / fma(den.x, den.x, den.y * den.y);
+    r.tau = make_double2(fma(-alpha.x, ib, 1.0), -alpha.y * ib);
     r.scal = make_double2(den.x * idd, -den.y * idd);
   }
   return r;
@@ -165,12 +191,17 @@ __host__ __device__ inline size_t sb_smem_bytes(int ld, int mr, bool yg, bool vg
 // The two row groups of a warp are summed with one shuffle, the eight warps'
 // sums in shared memory. The update of the columns has one form for every
 // column, a_c[r] -= a_j[r] s_c (s_c = scal w_c for c > j, 1 - scal for c = j,
-// 0 for c < j), so that the lanes of a warp do not diverge. T column j - 1 is
-// formed in iteration j by all warps, two rows each. The pivot column reaches
-// the threads of a row group through the warp's own shared-memory buffer (the
+// 0 for c < j), so that the lanes of a warp do not diverge. Rows go four at a
+// time (slots past the panel hold zeros), so that four loads of the pivot column
+// and four chains are in flight: with a check per row the two warps of a scheduler
+// waited for one load after another at large n. The pivot column reaches the threads of a row group through the warp's own shared-memory buffer (the
 // group's 16 threads share a warp). red/rowj: [2][8][16] / [2][16]; pvw
 // [8][2][MR]; dsm [16][16]; tsm [16]; T [16][17].
-template <int MR>
+// With VS (V in shared memory) the panel passes through V on its way between
+// global memory and the registers, so that a warp reads and writes 32 consecutive
+// rows of a column there; straight from the registers every access touches 16
+// columns (14 k cycles a panel, with T, at n = 274; 8 k now).
+template <int MR, bool VS>
 __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m, double2* V, double2* T,
                          double2* red, double2* rowj, double2* pvw, double2* dsm, double2* tsm) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -178,8 +209,19 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
   const int Mt = m / kNB;  // m is a multiple of 16: row slots t < Mt are inside the panel
   double2* pv = pvw + (size_t)wid * 2 * MR + (g & 1) * MR;  // this group's pivot buffer
   double2 col[MR];
+  double2* Ap = A + (size_t)c0 * ld + r0;  // element (r, c) of the panel at Ap[c ld + r]
+  if (VS) {
+#pragma unroll 2
+    for (int cc = wid; cc < kNB; cc += kNW)
+#pragma unroll 4
+      for (int r = lane; r < m; r += 32) V[pidx(r, cc)] = Ap[(size_t)cc * ld + r];
+    __syncthreads();
+  }
 #pragma unroll
-  for (int t = 0; t < MR; ++t) col[t] = t < Mt ? A[(size_t)(c0 + c) * ld + r0 + g + 16 * t] : make_double2(0, 0);
+  for (int t = 0; t < MR; ++t) {
+    const int r = g + 16 * t;
+    col[t] = t < Mt ? (VS ? V[pidx(r, c)] : Ap[(size_t)c * ld + r]) : make_double2(0, 0);
+  }
   // the group's rows of column 0 become the first pivot
   if (c == 0) {
 #pragma unroll
@@ -188,56 +230,52 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
   __syncwarp();
   for (int j = 0; j < kNB; ++j) {
     const int buf = j & 1;
-    // ---- partial sums over this thread's rows r > j (two chains)
-    double2 acc0 = make_double2(0, 0), acc1 = make_double2(0, 0);
-    if (g > j) {
-      const double2 aj = pv[0];
-      acc0.x = aj.x * col[0].x + aj.y * col[0].y;
-      acc0.y = aj.x * col[0].y - aj.y * col[0].x;
-    }
+    // ---- partial sums over this thread's rows r > j (four chains)
+    double2 sum[4];
 #pragma unroll
-    for (int t = 1; t < MR; ++t) {
-      if (t < Mt) {
-        const double2 aj = pv[t];
-        double2& a = (t & 1) ? acc1 : acc0;
-        a.x = fma(aj.x, col[t].x, fma(aj.y, col[t].y, a.x));
-        a.y = fma(aj.x, col[t].y, fma(-aj.y, col[t].x, a.y));
+    for (int u = 0; u < 4; ++u) sum[u] = make_double2(0, 0);
+    if (g > j) cfmac(sum[0], pv[0], col[0]);
+#pragma unroll
+    for (int t0 = 0; t0 < MR; t0 += 4) {
+      if (t0 < Mt) {
+        double2 aj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t0 + u > 0 && t0 + u < MR) aj[u] = pv[t0 + u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t0 + u > 0 && t0 + u < MR) cfmac(sum[u], aj[u], col[t0 + u]);
       }
     }
-    double2 acc = cadd(acc0, acc1);
+    double2 acc = cadd(cadd(sum[0], sum[1]), cadd(sum[2], sum[3]));
     acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16);
     acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
     if (lane < 16) red[(buf * 8 + wid) * 16 + c] = acc;
     if (g == j) rowj[buf * 16 + c] = col[0];  // row j = row group j, slot 0
     __syncthreads();
     double2 tq[8];
-    double xq[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      tq[q] = red[(buf * 8 + q) * 16 + c];
-      xq[q] = red[(buf * 8 + q) * 16 + j].x;
-    }
+    for (int q = 0; q < 8; ++q) tq[q] = red[(buf * 8 + q) * 16 + c];
     const double2 tot = cadd(cadd(cadd(tq[0], tq[1]), cadd(tq[2], tq[3])), cadd(cadd(tq[4], tq[5]), cadd(tq[6], tq[7])));
-    const double xn = ((xq[0] + xq[1]) + (xq[2] + xq[3])) + ((xq[4] + xq[5]) + (xq[6] + xq[7]));
+    const double xn = __shfl_sync(0xffffffffu, tot.x, (lane & 16) | j);  // column j's own sum
     const double2 alpha = rowj[buf * 16 + j], rj = rowj[buf * 16 + c];
-    // T column j - 1 (its dots are complete now): T[0:j-1, j-1] = -tau T d,
-    // rows 2 wid and 2 wid + 1
-    if (j >= 1) {
-      const int jj = j - 1, l = 2 * wid + (lane >> 4);
-      double2 p = c >= l && c < jj ? cmul(T[l * 17 + c], dsm[jj * 16 + c]) : make_double2(0, 0);
-      p.x = sum16(p.x);
-      p.y = sum16(p.y);
-      const double2 tj = tsm[jj];
-      if (c == 0) T[l * 17 + jj] = l < jj ? cmul(make_double2(-tj.x, -tj.y), p) : (l == jj ? tj : make_double2(0, 0));
-    }
     const Refl R = make_refl(alpha, xn);
     // w_c = conj(tau) v^H a_c (v = (1; scal a_j)); a_c -= v w_c
     const double2 w = cmul(cconj(R.tau), cadd(rj, cmulc(R.scal, tot)));
     const double2 sw = c > j ? cmul(R.scal, w) : (c == j ? make_double2(1.0 - R.scal.x, -R.scal.y) : make_double2(0, 0));
-    if (g > j) col[0] = csub(col[0], cmul(pv[0], sw));
+    if (g > j) cfms(col[0], pv[0], sw);
 #pragma unroll
-    for (int t = 1; t < MR; ++t)
-      if (t < Mt) col[t] = csub(col[t], cmul(pv[t], sw));
+    for (int t0 = 0; t0 < MR; t0 += 4) {
+      if (t0 < Mt) {
+        double2 aj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t0 + u > 0 && t0 + u < MR) aj[u] = pv[t0 + u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (t0 + u > 0 && t0 + u < MR) cfms(col[t0 + u], aj[u], sw);
+      }
+    }
     if (g == j) col[0] = c > j ? csub(col[0], w) : (c == j ? make_double2(R.beta, 0.0) : col[0]);
     if (g == 0 && c < j) dsm[j * 16 + c] = cadd(cconj(rj), cmul(R.scal, cconj(tot)));  // v_c^H v_j
     if (tid == 0) tsm[j] = R.tau;
@@ -245,28 +283,51 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
     __syncwarp();
     if (j + 1 < kNB && c == j + 1) {
 #pragma unroll
-      for (int t = 0; t < MR; ++t) pv[t] = col[t];
+      for (int t = 0; t < MR; ++t)
+        if ((t & ~3) < Mt) pv[t] = col[t];
     }
     __syncwarp();
   }
   __syncthreads();
-  if (wid == 0) {  // last T column
-    const int jj = kNB - 1;
-    double2 sacc = make_double2(0, 0);
-    if (lane < jj)
-      for (int q = lane; q < jj; ++q) sacc = cadd(sacc, cmul(T[lane * 17 + q], dsm[jj * 16 + q]));
-    const double2 tj = tsm[jj];
-    if (lane < jj) T[lane * 17 + jj] = cmul(make_double2(-tj.x, -tj.y), sacc);
-    if (lane == jj) T[jj * 17 + jj] = tj;
-  }
   // R and the reflectors back in place (band and back-transform); V explicit
-  // in shared memory
+  // (unit diagonal, zeros above it)
+  if (VS) {
 #pragma unroll
-  for (int t = 0; t < MR; ++t) {
-    const int r = g + 16 * t;
-    if (t < Mt) {
-      A[(size_t)(c0 + c) * ld + r0 + r] = col[t];
-      V[pidx(r, c)] = r < c ? make_double2(0, 0) : (r == c ? make_double2(1, 0) : col[t]);
+    for (int t = 0; t < MR; ++t)
+      if (t < Mt) V[pidx(g + 16 * t, c)] = col[t];
+    __syncthreads();
+#pragma unroll 2
+    for (int cc = wid; cc < kNB; cc += kNW)
+#pragma unroll 4
+      for (int r = lane; r < m; r += 32) Ap[(size_t)cc * ld + r] = V[pidx(r, cc)];
+    __syncthreads();
+    if (g <= c) V[pidx(g, c)] = make_double2(g == c ? 1.0 : 0.0, 0.0);
+  } else {
+#pragma unroll
+    for (int t = 0; t < MR; ++t) {
+      const int r = g + 16 * t;
+      if (t < Mt) {
+        Ap[(size_t)c * ld + r] = col[t];
+        V[pidx(r, c)] = r < c ? make_double2(0, 0) : (r == c ? make_double2(1, 0) : col[t]);
+      }
+    }
+  }
+  // T[0:j, j] = -tau_j T[0:j, 0:j] (v_0 .. v_{j-1})^H v_j (zlarft), column after
+  // column: lane i of warp 0 keeps row i, its two halves take every other term
+  if (wid == 0) {
+    const int i = lane & 15, h = lane >> 4;
+    double2 row[kNB];
+#pragma unroll
+    for (int j = 0; j < kNB; ++j) {
+      double2 p = make_double2(0, 0);
+#pragma unroll
+      for (int q = 0; q < kNB; ++q)
+        if (q < j && (q & 1) == h) cfma(p, row[q], dsm[j * 16 + q]);
+      p.x += __shfl_xor_sync(0xffffffffu, p.x, 16);
+      p.y += __shfl_xor_sync(0xffffffffu, p.y, 16);
+      const double2 tj = tsm[j];
+      row[j] = i < j ? cmul(make_double2(-tj.x, -tj.y), p) : (i == j ? tj : make_double2(0, 0));
+      if (h == 0) T[i * 17 + j] = row[j];
     }
   }
   __syncthreads();
@@ -287,7 +348,6 @@ __device__ void pass_y(const double2* __restrict__ A, int ld, int r0, int Mt, co
     double cr[2][2], ci[2][2];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb) cr[nb][0] = cr[nb][1] = ci[nb][0] = ci[nb][1] = 0.0;
-    double2 a[4], an[4];
     auto load_a = [&](int J, double2 (&f)[4]) {
 #pragma unroll
       for (int kb = 0; kb < 4; ++kb) {
@@ -298,34 +358,51 @@ __device__ void pass_y(const double2* __restrict__ A, int ld, int r0, int Mt, co
           f[kb] = cconj(A[(size_t)row * ld + col]);
       }
     };
-    double2 bf[4][2], bfn[4][2];
-    auto load_b = [&](int J, double2 (&f)[4][2]) {
+    if (PF) {
+      double2 a[4], an[4], bf[4][2], bfn[4][2];
+      auto load_b = [&](int J, double2 (&f)[4][2]) {
 #pragma unroll
-      for (int kb = 0; kb < 4; ++kb)
+        for (int kb = 0; kb < 4; ++kb)
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) f[kb][nb] = V[pidx(16 * J + 4 * kb + gk, 8 * nb + gr)];
-    };
-    load_a(0, a);
-    if (PF) load_b(0, bf);
-    for (int J = 0; J < Mt; ++J) {
-      if (J + 1 < Mt) {
-        load_a(J + 1, an);
-        if (PF) load_b(J + 1, bfn);
-      }
-#pragma unroll
-      for (int kb = 0; kb < 4; ++kb) {
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-          const double2 b = PF ? bf[kb][nb] : V[pidx(16 * J + 4 * kb + gk, 8 * nb + gr)];
-          cmma(cr[nb], ci[nb], a[kb], b);
+          for (int nb = 0; nb < 2; ++nb) f[kb][nb] = V[pidx(16 * J + 4 * kb + gk, 8 * nb + gr)];
+      };
+      load_a(0, a);
+      load_b(0, bf);
+      for (int J = 0; J < Mt; ++J) {
+        if (J + 1 < Mt) {
+          load_a(J + 1, an);
+          load_b(J + 1, bfn);
         }
-      }
 #pragma unroll
-      for (int kb = 0; kb < 4; ++kb) {
-        a[kb] = an[kb];
-        if (PF) {
+        for (int kb = 0; kb < 4; ++kb)
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb) cmma(cr[nb], ci[nb], a[kb], bf[kb][nb]);
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb) {
+          a[kb] = an[kb];
 #pragma unroll
           for (int nb = 0; nb < 2; ++nb) bf[kb][nb] = bfn[kb][nb];
+        }
+      }
+    } else {
+      // the blocks J + kAhead, ... are on their way while J is multiplied
+      constexpr int kAhead = 3;
+      double2 a[kAhead + 1][4];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (u < Mt) load_a(u, a[u]);
+      for (int J0 = 0; J0 < Mt; J0 += kAhead + 1) {
+#pragma unroll
+        for (int u = 0; u <= kAhead; ++u) {
+          const int J = J0 + u;
+          if (J < Mt) {
+            if (J + kAhead < Mt) load_a(J + kAhead, a[(u + kAhead) % (kAhead + 1)]);
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb)
+#pragma unroll
+              for (int nb = 0; nb < 2; ++nb)
+                cmma(cr[nb], ci[nb], a[u][kb], V[pidx(16 * J + 4 * kb + gk, 8 * nb + gr)]);
+          }
         }
       }
     }
@@ -456,7 +533,7 @@ __global__ void __launch_bounds__(kThr, 1) sb_kernel(const EigItem* __restrict__
 
   for (int c0 = 0; c0 + kNB < ld; c0 += kNB) {
     const int r0 = c0 + kNB, m = ld - r0, Mt = m / kNB;
-    panel_qr<MR>(A, ld, c0, r0, m, S.V, S.T, S.part, S.rowj, S.pvw, S.M, S.taus);
+    panel_qr<MR, !KVG>(A, ld, c0, r0, m, S.V, S.T, S.part, S.rowj, S.pvw, S.M, S.taus);
     // T into the free upper tile (rows c0.., columns r0..) for the back-transform
     for (int idx = tid; idx < kNB * kNB; idx += kThr) {
       const int i = idx % kNB, j = idx / kNB;
@@ -645,53 +722,12 @@ __device__ __forceinline__ void publish(int* flag, int v, int lane) {
   }
 }
 
-// acc += a b, acc += conj(a) b, acc -= a b, acc -= a conj(b)
-__device__ __forceinline__ void cfma(double2& acc, double2 a, double2 b) {
-  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
-}
-__device__ __forceinline__ void cfmac(double2& acc, double2 a, double2 b) {
-  acc.x = fma(a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-__device__ __forceinline__ void cfms(double2& acc, double2 a, double2 b) {
-  acc.x = fma(-a.x, b.x, fma(a.y, b.y, acc.x));
-  acc.y = fma(-a.x, b.y, fma(-a.y, b.x, acc.y));
-}
-__device__ __forceinline__ void cfmsc(double2& acc, double2 a, double2 b) {
-  acc.x = fma(-a.x, b.x, fma(-a.y, b.y, acc.x));
-  acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
-}
 __device__ __forceinline__ double2 shfl2(double2 v, int src) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 __device__ __forceinline__ void add_halves(double2& v) {
   v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
   v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
-}
-
-// make_refl on a short dependency chain: 1 / beta is the reciprocal square root,
-// beta its product with the sum corrected by one Newton step (to the rounding
-// of a square root)
-__device__ __forceinline__ Refl make_refl_fast(double2 alpha, double xn) {
-  Refl r;
-  if (xn == 0.0 && alpha.y == 0.0) {
-    r.tau = make_double2(0, 0);
-    r.beta = alpha.x;
-    r.scal = make_double2(1, 0);
-  } else {
-    const double s2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn));
-    const double rs = rsqrt(s2);
-    double nrm = s2 * rs;
-    nrm = fma(0.5 * rs, fma(-nrm, nrm, s2), nrm);
-    r.beta = -copysign(nrm, alpha.x);
-    const double ib = -copysign(rs, alpha.x);
-    const double2 den = make_double2(alpha.x - r.beta, alpha.y);
-    const double idd = 1.0 / fma(den.x, den.x, den.y * den.y);
-    r.tau = make_double2(fma(-alpha.x, ib, 1.0), -alpha.y * ib);
-    r.scal = make_double2(den.x * idd, -den.y * idd);
-  }
-  return r;
 }
 
 // KBG: the band in the item's work area of the reflector buffer (ld >
@@ -758,7 +794,7 @@ __global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restr
       double2* cs = B - kBandLd + 1;
       const double2 xi = cs[i];
       const double xx = sum16(i >= 1 ? fma(xi.x, xi.x, xi.y * xi.y) : 0.0);
-      const Refl Rf = make_refl_fast(cs[0], xx);
+      const Refl Rf = make_refl(cs[0], xx);
       __syncwarp();
       if (h == 0) {
         const double2 v = i == 0 ? make_double2(1, 0) : cmul(xi, Rf.scal);
@@ -838,7 +874,7 @@ __global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restr
         // the first column x in both halves
         const double2 x = shfl2(e[0], i);
         const double xx = sum16(i >= 1 ? fma(x.x, x.x, x.y * x.y) : 0.0);
-        const Refl Rf = make_refl_fast(shfl2(x, 0), xx);
+        const Refl Rf = make_refl(shfl2(x, 0), xx);
 #pragma unroll
         for (int cc = 1; cc < 8; ++cc) cfmsc(e[cc], tu, vc[cc]);
         double2* nx = sl + ((j + 1) & 1) * kSlot;
@@ -903,7 +939,7 @@ __global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restr
 // same up to 148 matrices, 3-5 % slower solver beyond). Measured on a B200 against
 // one kernel with divisions in the Sturm chain, one thread per eigenvalue cluster
 // and four factor arrays: 296 matrices of n = 274 with 17 vectors 0.67 -> 0.12 +
-// 0.22 ms, 148 of n = 570 with 25 vectors 2.37 -> 0.16 + 0.42 ms.
+// 0.21 ms, 148 of n = 570 with 25 vectors 2.37 -> 0.17 + 0.44 ms.
 constexpr int kTriThr = 256, kTriVecThr = 64;
 
 inline size_t tri_smem_bytes(int n, int nval) {
