@@ -136,9 +136,12 @@ bool overlap_tiles(int ncd_max, int nvd_max, int n, int npw, int& cchunk, int& v
 // (0: no shape fits).
 int overlap_tile_candidates(int ncd_max, int nvd_max, int n, int npw, int* cc, int* vc, int maxc);
 // FP64 contraction on the FP64 tensor cores (contract64.cu); T transitions,
-// ws: contract64_workspace_bytes
-cudaError_t launch_contract64(const ContractArgs& a, long long T, double* ws, cudaStream_t st);
-size_t contract64_workspace_bytes(const ContractArgs& a, long long T);
+// table: the line shapes are tabulated first (contract64_wants_table: where that
+// pays and fits), ws: contract64_workspace_bytes; nlaunch: kernels launched
+cudaError_t launch_contract64(const ContractArgs& a, long long T, void* ws, bool table, int& nlaunch,
+                              cudaStream_t st);
+size_t contract64_workspace_bytes(const ContractArgs& a, long long T, bool table);
+bool contract64_wants_table(const ContractArgs& a, long long T);
 // FP64 contraction with the principal-value sums (acc_pv, one channel)
 cudaError_t launch_contract_pv(const ContractArgs& a, cudaStream_t st);
 // frequencies per transition range (ContractArgs::trange)

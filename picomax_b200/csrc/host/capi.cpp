@@ -1381,11 +1381,17 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
       CK(pmx::dev::launch_contract_pv(ca, st));
       ctx->launches += 1;
     } else if (precision == PMX_PREC_FP64) {
-      const size_t wsb = pmx::dev::contract64_workspace_bytes(ca, Tn);
-      CK(ctx->c64ws.ensure(wsb));
+      // without the memory for the table of line shapes the kernel forms them itself
+      bool table = pmx::dev::contract64_wants_table(ca, Tn);
+      if (table && ctx->c64ws.ensure(pmx::dev::contract64_workspace_bytes(ca, Tn, true)) != cudaSuccess) {
+        cudaGetLastError();
+        table = false;
+      }
+      CK(ctx->c64ws.ensure(pmx::dev::contract64_workspace_bytes(ca, Tn, table)));
+      int nl = 0;
       KTime kt(ctx, "contract_f64");
-      CK(pmx::dev::launch_contract64(ca, Tn, ctx->c64ws.as<double>(), st));
-      ctx->launches += wsb ? 2 : 1;
+      CK(pmx::dev::launch_contract64(ca, Tn, ctx->c64ws.ptr, table, nl, st));
+      ctx->launches += nl;
     } else {
       int nl = 0;
       CK(ctx->mixws.ensure(std::max<size_t>(pmx::dev::mixed_workspace_bytes(ca, Tn), 16)));
