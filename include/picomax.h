@@ -173,9 +173,10 @@ int pmx_ctx_mixed_mmas(const pmx_ctx* ctx, long long* mmas);
  * overlaps); the fastest is kept for the rest of the context's life. No
  * reference counterpart. */
 int pmx_ctx_set_autotune(pmx_ctx* ctx, int on);
-/* Fixes the eigensolver schedule (0 = direct loads, then the prefetch and
- * shared-memory-partials schedules the matrix size allows; an index beyond
- * the last one means the last) for every later batch; -1 returns to the
+/* Fixes the eigensolver schedule (0 = the two-stage solver where it applies,
+ * n >= 96, then the one-stage schedules the matrix size allows: direct loads,
+ * prefetch rings, shared-memory partials; an index beyond the last one means
+ * the last) for every later batch; -1 returns to the
  * autotuner. For tests that compare the schedules. No reference counterpart. */
 int pmx_ctx_set_schedule(pmx_ctx* ctx, int schedule);
 /* The autotuner's choices and trial times as JSON text (NUL-terminated,

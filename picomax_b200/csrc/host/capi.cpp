@@ -428,14 +428,18 @@ DevCrystal upload_crystal(pmx_ctx* c, const pmx_problem* P, int force_spinor) {
   return d;
 }
 
-// Eigensolver dispatch. Where the two-stage solver applies (matrices too
-// large for the shared-memory-resident one-stage kernel, padded size <= 832,
-// and no export of the one-stage reduction for the adjoint) it is schedule 0
-// and the one-stage schedules follow; otherwise only the one-stage schedules
-// are offered. A launch's items then carry the padded leading dimension and
-// a slot of the band reflector buffer (ctx rbuf).
+// Eigensolver dispatch. Where the two-stage solver applies (n from 96 to a padded
+// size of 1216, and no export of the one-stage reduction for the adjoint) it is
+// schedule 0 and the one-stage schedules follow; otherwise only the one-stage
+// schedules are offered. A launch's items then carry the padded leading dimension
+// and a slot of the band reflector buffer (ctx rbuf).
+// The line at 96, measured on a B200 (two-stage / one-stage, whose matrix fits in
+// shared memory up to n = 153): 433 matrices of n = 81 1.19 / 1.04 ms; 122 of
+// n = 96 0.51 / 0.60; n = 113 122 0.71 / 0.81, 433 1.77 / 2.42, 1025 3.89 / 5.64;
+// 1025 of n = 137 4.82 / 9.97; 433 of n = 153 2.58 / 5.00 ms.
+constexpr int kTwoStageMin = 96;
 bool use_two_stage(int max_n, bool tri) {
-  return !tri && max_n > pmx::dev::heev_smem_max_n() && pmx::dev::heev2_supported(max_n);
+  return !tri && max_n >= kTwoStageMin && pmx::dev::heev2_supported(max_n);
 }
 int eig_variants(int max_n, int max_nval, bool tri) {
   return (use_two_stage(max_n, tri) ? 1 : 0) + pmx::dev::heev_variants(max_n, max_nval);

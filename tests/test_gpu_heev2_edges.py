@@ -7,7 +7,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-CASES = [(154, 1, "dense"), (160, 7, "dense"), (161, 8, "banded"), (175, 9, "dense"), (176, 16, "blocks"),
+CASES = [(96, 8, "dense"), (97, 3, "banded"), (112, 33, "blocks"), (113, 9, "diagonal"), (128, 20, "dense"),
+         (153, 2, "dense"), (154, 1, "dense"), (160, 7, "dense"), (161, 8, "banded"), (175, 9, "dense"), (176, 16, "blocks"),
          (177, 17, "diagonal"), (200, 31, "dense"), (256, 32, "banded"), (273, 33, "dense"), (289, 5, "blocks"),
          (300, 40, "diagonal"), (400, 3, "dense"), (416, 24, "dense"), (417, 24, "dense"), (433, 65, "blocks"),
          (160, 12, "zero"), (818, 6, "banded"), (180, 180, "dense")]
