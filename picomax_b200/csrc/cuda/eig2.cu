@@ -654,8 +654,8 @@ __global__ void __launch_bounds__(kThr, 1) sb_kernel(const EigItem* __restrict__
 // (one base address a step), sums are fused multiply-adds, a reflector takes one
 // rsqrt and one reciprocal, both halves of the warp keep the first column so that
 // its norm takes four shuffles, and the sweep's first reflector is D's work.
-// Measured on a B200: 296 matrices of n = 274 2.31 -> 1.58 ms, 148 of n = 570
-// (band in global memory) 4.84 -> 4.02 ms, against tasks that waited for whole
+// Measured on a B200: 296 matrices of n = 274 2.31 -> 1.50 ms, 148 of n = 570
+// (band in global memory) 4.84 -> 3.9 ms, against tasks that waited for whole
 // tasks of the sweep before, with a barrier per step and checks of every row and
 // column (1770 warp instructions a task, now 1000 with the polls).
 constexpr int kBandLd = 2 * kNB;
@@ -692,12 +692,12 @@ __device__ __forceinline__ long long global_ns() {
   return t;
 }
 
-// Waits until *flag >= need: a few polls at once, then one every ~kPollNs so
+// Waits until *flag >= need: kSpin polls at once, then one every ~kPollNs so
 // that a waiting warp leaves the issue slots to the warps that work. Gives up,
 // and sets *err, after limit_ns, after 2^28 polls, or at once when another warp
 // has given up already.
-constexpr unsigned kPollNs = 20;
-constexpr int kSpin = 8;
+constexpr unsigned kPollNs = 40;
+constexpr int kSpin = 1;
 __device__ __forceinline__ void wait_progress(const int* flag, int need, int* err, long long limit_ns) {
 #pragma unroll 1
   for (int k = 0; k < kSpin; ++k)
@@ -758,7 +758,9 @@ __global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restr
   __syncthreads();
   const int i = lane & 15, h = lane >> 4;
   const int pair = wid >> 1;
-  const bool ewarp = (wid & 1) != 0;  // E (bulge) warp, else D (diagonal block) warp
+  // E (bulge) warp, else D (diagonal block) warp: in every other two pairs the roles
+  // are swapped, so that each of the four schedulers (warp mod 4) has two E warps
+  const bool ewarp = ((wid ^ (pair >> 1)) & 1) != 0;
   double2* wv = wsm + wid * kSlot;
   double2* sl = slots + pair * 2 * kSlot;
   const long long limit = it.wait_ns > 0 ? it.wait_ns : kWaitNs;
