@@ -516,43 +516,46 @@ namespace dev {
 // ------------------------------------------------------------ macroscopic eps
 // eps_M(q, w) = 1 / [eps^-1]_00 with eps_mn = delta_mn + chi^LL_mn and the
 // n > m half filled by conj(eps_nm), as in the reference's post-processing
-// (include/matlab_wrapper/+picomax/+eps/macroscopic.m:13-29, :79). One warp
-// per (q, w): Gaussian elimination with partial pivoting of eps x = e_0 in
-// shared memory; [eps^-1]_00 = x_0.
+// (include/matlab_wrapper/+picomax/+eps/macroscopic.m:13-29, :79). 1 / [eps^-1]_00
+// is the Schur complement of eps[1:, 1:]: with vector 0 last, Gaussian elimination
+// with partial pivoting among the other rows leaves it in the last diagonal
+// element, and no back substitution is needed. One CTA per (q, w), the matrix in
+// shared memory, lanes over columns and warps over rows: bound by the latency of
+// the n steps, so that several CTAs share an SM (four of 59 vectors; four warps of
+// one CTA had a matrix each before, with a serial back substitution). Measured on a
+// B200, 2000 frequencies: 59 vectors 2.06 -> 0.58 ms, 27 vectors 0.138 -> 0.089 ms, 15
+// vectors 0.058 -> 0.046 ms.
 __global__ void __launch_bounds__(128) epsm_kernel(const double* __restrict__ re, const double* __restrict__ im,
-                                                   int neps, int nq, int nf, double2* __restrict__ out) {
+                                                   int neps, int nf, double2* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int job = blockIdx.x * (blockDim.x >> 5) + w;
-  if (job >= nq * nf) return;
-  const int q = job / nf, f = job % nf;
-  const int n = neps, ld = n + 1;
-  double2* E = reinterpret_cast<double2*>(smraw) + (size_t)w * n * ld;  // row-major, column n = rhs
-  const int np = n * (n + 1) / 2;
+  double2* E = reinterpret_cast<double2*>(smraw);  // [n][n], row and column m at (m + n - 1) % n
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int job = blockIdx.x, q = job / nf, f = job % nf;
+  const int n = neps, np = n * (n + 1) / 2;
   // chi LL block: [i=0][j=0][q][pair][f]
-  for (int idx = lane; idx < n * n; idx += 32) {
-    const int r = idx / n, c = idx % n;
-    const int m = r > c ? r : c, nn = r > c ? c : r;
-    const size_t o = ((size_t)q * np + (size_t)m * (m + 1) / 2 + nn) * nf + f;
-    double2 v = make_double2(re[o], im[o]);
-    if (r < c) v.y = -v.y;  // eps_nm = conj(eps_mn) above the diagonal
-    if (r == c) v.x += 1.0;
-    E[r * ld + c] = v;
-  }
-  for (int r = lane; r < n; r += 32) E[r * ld + n] = make_double2(r == 0 ? 1.0 : 0.0, 0.0);
-  __syncwarp();
-  for (int k = 0; k < n; ++k) {
-    // pivot search (lane-strided, then warp argmax)
+  for (int r = wid; r < n; r += nw)
+    for (int c = lane; c <= r; c += 32) {
+      const size_t o = ((size_t)q * np + (size_t)r * (r + 1) / 2 + c) * nf + f;
+      double2 v = make_double2(re[o], im[o]);
+      const int ri = r == 0 ? n - 1 : r - 1, ci = c == 0 ? n - 1 : c - 1;
+      if (r == c) v.x += 1.0;
+      E[ri * n + ci] = v;
+      if (r != c) E[ci * n + ri] = cconj(v);  // eps_nm = conj(eps_mn) above the diagonal
+    }
+  __syncthreads();
+  for (int k = 0; k < n - 1; ++k) {
+    // pivot among rows k .. n - 2, the same search in every warp
     double best = -1.0;
     int bi = k;
-    for (int r = k + lane; r < n; r += 32) {
-      const double2 v = E[r * ld + k];
+    for (int r = k + lane; r < n - 1; r += 32) {
+      const double2 v = E[r * n + k];
       const double a = v.x * v.x + v.y * v.y;
       if (a > best) {
         best = a;
         bi = r;
       }
     }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const double ob = __shfl_xor_sync(0xffffffffu, best, o);
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
@@ -561,46 +564,35 @@ __global__ void __launch_bounds__(128) epsm_kernel(const double* __restrict__ re
         bi = oi;
       }
     }
-    if (bi != k)
-      for (int c = lane; c <= n; c += 32) {
-        const double2 t = E[k * ld + c];
-        E[k * ld + c] = E[bi * ld + c];
-        E[bi * ld + c] = t;
+    if (bi != k) {
+      __syncthreads();  // every warp has searched
+      for (int c = k + threadIdx.x; c < n; c += blockDim.x) {
+        const double2 t = E[k * n + c];
+        E[k * n + c] = E[bi * n + c];
+        E[bi * n + c] = t;
       }
-    __syncwarp();
-    const double2 p = E[k * ld + k];
+      __syncthreads();
+    }
+    const double2 p = E[k * n + k];
     const double pd = p.x * p.x + p.y * p.y;
     const double2 inv = make_double2(p.x / pd, -p.y / pd);
-    for (int r = k + 1; r < n; ++r) {
-      const double2 fct = cmul(E[r * ld + k], inv);
-      for (int c = k + lane; c <= n; c += 32) E[r * ld + c] = csub(E[r * ld + c], cmul(fct, E[k * ld + c]));
+    for (int r = k + 1 + wid; r < n; r += nw) {
+      const double2 fct = cmul(E[r * n + k], inv);
+      for (int c = k + 1 + lane; c < n; c += 32) E[r * n + c] = csub(E[r * n + c], cmul(fct, E[k * n + c]));
     }
-    __syncwarp();
+    __syncthreads();
   }
-  if (lane == 0) {
-    // back substitution for x_0 only needs the full solve; do it serially
-    double2 x[64];
-    for (int r = n - 1; r >= 0; --r) {
-      double2 s = E[r * ld + n];
-      for (int c = r + 1; c < n; ++c) s = csub(s, cmul(E[r * ld + c], x[c]));
-      const double2 d = E[r * ld + r];
-      const double dd = d.x * d.x + d.y * d.y;
-      x[r] = cmul(s, make_double2(d.x / dd, -d.y / dd));
-    }
-    const double2 x0 = x[0];
-    const double xx = x0.x * x0.x + x0.y * x0.y;
-    out[job] = make_double2(x0.x / xx, -x0.y / xx);
-  }
+  if (threadIdx.x == 0) out[job] = E[n * n - 1];
 }
 
 cudaError_t launch_epsm(const double* re, const double* im, int neps, int nq, int nf, double2* out, cudaStream_t st) {
   if (neps > 64 || neps < 1) return cudaErrorInvalidValue;
-  const int warps = 4;
-  const size_t smem = (size_t)warps * neps * (neps + 1) * sizeof(double2);
+  const size_t smem = (size_t)neps * neps * sizeof(double2);
   cudaError_t e = cudaFuncSetAttribute(epsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int jobs = nq * nf;
-  epsm_kernel<<<(jobs + warps - 1) / warps, 32 * warps, smem, st>>>(re, im, neps, nq, nf, out);
+  // warps per matrix: one row pass of the lanes per warp up to 32 vectors
+  const int thr = neps <= 16 ? 32 : (neps <= 32 ? 64 : 128);
+  epsm_kernel<<<nq * nf, thr, smem, st>>>(re, im, neps, nf, out);
   return cudaGetLastError();
 }
 
