@@ -677,6 +677,27 @@ cudaError_t launch_resolvent(const ResolventArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
+__global__ void sub_kernel(const double2* __restrict__ a, const double2* __restrict__ b, double2* __restrict__ out,
+                           long long count, bool add) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += (long long)gridDim.x * blockDim.x) {
+    const double2 v = csub(a[i], b[i]);
+    out[i] = add ? cadd(out[i], v) : v;
+  }
+}
+static cudaError_t run_sub(const double2* a, const double2* b, double2* out, long long count, bool add,
+                           cudaStream_t st) {
+  if (count <= 0) return cudaSuccess;
+  sub_kernel<<<(int)std::min<long long>((count + 255) / 256, 148LL * 16), 256, 0, st>>>(a, b, out, count, add);
+  return cudaGetLastError();
+}
+cudaError_t launch_sub(const double2* a, const double2* b, double2* out, long long count, cudaStream_t st) {
+  return run_sub(a, b, out, count, false, st);
+}
+cudaError_t launch_add_sub(const double2* a, const double2* b, double2* y, long long count, cudaStream_t st) {
+  return run_sub(a, b, y, count, true, st);
+}
+
 // ------------------------------------------------------- pair accumulators
 namespace {
 constexpr int kHT = 16, kHJ = 8;

@@ -1045,9 +1045,12 @@ __global__ void __launch_bounds__(kTriVecThr) tri_vec_kernel(const EigItem* __re
 // one CTA per matrix with a barrier per sweep and panel columns on the CUDA cores:
 // 296 matrices of n = 274 with 17 vectors 1.25 -> 0.97 ms (1184: 4.9 -> 2.8 ms),
 // 148 of n = 570 with 25 vectors 6.1 -> 3.6 ms.
+// ADJ applies Q2^H instead (the adjoint's resolvent): groups, steps and reflectors in
+// the opposite order, with the conjugate of tau, the window moving up.
 constexpr int kBackG = 16;     // sweeps per group
 constexpr int kBackLanes = 4;  // lanes per vector
 
+template <bool ADJ>
 __global__ void __launch_bounds__(32, 16) band_back_kernel(const EigItem* __restrict__ items,
                                                       const double2* __restrict__ rbuf, double2* __restrict__ zbuf,
                                                       const int* __restrict__ info) {
@@ -1080,19 +1083,21 @@ __global__ void __launch_bounds__(32, 16) band_back_kernel(const EigItem* __rest
     cp_async_commit();
   };
   auto load = [&](int r) { return r + h < n ? z[r] : make_double2(0, 0); };
-  for (int S = (ld - 2) / kBackG * kBackG; S >= 0; S -= kBackG) {
+  const int last = (ld - 2) / kBackG * kBackG;
+  for (int g = 0; g <= last; g += kBackG) {
+    const int S = ADJ ? g : last - g;
     const int nj = sweep_steps(ld, S);
     double2 w[kM];
-    stage(0, S, 0);
+    int p0 = ADJ ? S + kNB * (nj - 1) : S;  // first row of the window
+    stage(0, S, ADJ ? nj - 1 : 0);
 #pragma unroll
-    for (int m = 0; m < kM; ++m) w[m] = load(S + G * m);
-    int p0 = S;
-    for (int j = 0; j < nj; ++j, p0 += kNB) {
+    for (int m = 0; m < kM; ++m) w[m] = load(p0 + G * m);
+    for (int u = 0; u < nj; ++u, p0 += ADJ ? -kNB : kNB) {
       double2 wn[kHalf];
-      if (j + 1 < nj) {
-        stage((j + 1) & 1, S, j + 1);
+      if (u + 1 < nj) {
+        stage((u + 1) & 1, S, ADJ ? nj - 2 - u : u + 1);
 #pragma unroll
-        for (int m = 0; m < kHalf; ++m) wn[m] = load(p0 + 2 * kNB + G * m);
+        for (int m = 0; m < kHalf; ++m) wn[m] = load(p0 + (ADJ ? -kNB : 2 * kNB) + G * m);
         cp_async_wait<1>();
       } else {
 #pragma unroll
@@ -1100,11 +1105,12 @@ __global__ void __launch_bounds__(32, 16) band_back_kernel(const EigItem* __rest
         cp_async_wait<0>();
       }
       __syncwarp();
-      const double2* v = sv + (j & 1) * kBackG * kSt + h + G - 1;
-      const double2* tv = st + (j & 1) * kBackG;
+      const double2* v = sv + (u & 1) * kBackG * kSt + h + G - 1;
+      const double2* tv = st + (u & 1) * kBackG;
 #pragma unroll
-      for (int t = kBackG - 1; t >= 0; --t) {
+      for (int tt = 0; tt < kBackG; ++tt) {
         // rows t + 1 .. t + 16 of the window: entry q = G m + h - (t + 1)
+        const int t = ADJ ? tt : kBackG - 1 - tt;
         constexpr int kE = kNB / G + 1;
         const int m0 = (t + 1) / G, ne = (t + kNB) / G - m0 + 1;
         double2 ve[kE], d0 = make_double2(0, 0), d1 = make_double2(0, 0);
@@ -1121,24 +1127,30 @@ __global__ void __launch_bounds__(32, 16) band_back_kernel(const EigItem* __rest
           d.x += __shfl_xor_sync(0xffffffffu, d.x, o);
           d.y += __shfl_xor_sync(0xffffffffu, d.y, o);
         }
-        d = cmul(tv[t], d);
+        d = ADJ ? cmulc(tv[t], d) : cmul(tv[t], d);
 #pragma unroll
         for (int e = 0; e < kE; ++e)
           if (e < ne) cfms(w[m0 + e], ve[e], d);
       }
       __syncwarp();  // the staged reflectors have been read
+      // the half of the window that this group is done with
 #pragma unroll
       for (int m = 0; m < kHalf; ++m) {
-        const int r = p0 + G * m;
-        if (own && r + h < n) z[r] = w[m];
-        w[m] = w[m + kHalf];
-        w[m + kHalf] = wn[m];
+        const int out = ADJ ? m + kHalf : m, r = p0 + G * out;
+        if (own && r + h < n) z[r] = w[out];
+        if (ADJ) {
+          w[m + kHalf] = w[m];
+          w[m] = wn[m];
+        } else {
+          w[m] = w[m + kHalf];
+          w[m + kHalf] = wn[m];
+        }
       }
     }
 #pragma unroll
     for (int m = 0; m < kHalf; ++m) {
-      const int r = p0 + G * m;
-      if (own && r + h < n) z[r] = w[m];
+      const int out = ADJ ? m + kHalf : m, r = p0 + G * out;
+      if (own && r + h < n) z[r] = w[out];
     }
   }
 }
@@ -1163,7 +1175,8 @@ inline size_t panel_back_smem(int ld) {
   return sizeof(double2) * ((size_t)ld * panel_ldz<NB>() + 2 * kNB * panel_ldz<NB>() + kNB * 17 + (kNW / NB) * kNB * 8 * NB);
 }
 
-template <int NB>
+// ADJ applies Q1^H: the panels forward, with T^H.
+template <int NB, bool ADJ>
 __global__ void __launch_bounds__(kThr, 2) panel_back_kernel(const EigItem* __restrict__ items,
                                                            const double2* __restrict__ hbuf,
                                                            double2* __restrict__ zbuf, const int* __restrict__ info) {
@@ -1187,7 +1200,8 @@ __global__ void __launch_bounds__(kThr, 2) panel_back_kernel(const EigItem* __re
     Z[r * kLdz + k] = k < nv && r < n ? zg[(size_t)k * n + r] : make_double2(0, 0);
   }
   const int nb = wid % NB, kg = wid / NB;  // this warp's vectors and share of the rows in V^H Z
-  for (int c0 = ld - 2 * kNB; c0 >= 0; c0 -= kNB) {
+  for (int pc = 0; pc <= ld - 2 * kNB; pc += kNB) {
+    const int c0 = ADJ ? pc : ld - 2 * kNB - pc;
     const int r0 = c0 + kNB, m = ld - r0;
     const double2* Vp = A + (size_t)c0 * ld + r0;  // column i at Vp + i ld
     if (tid < kNB * kNB) {
@@ -1227,7 +1241,10 @@ __global__ void __launch_bounds__(kThr, 2) panel_back_kernel(const EigItem* __re
     for (int idx = tid; idx < kNB * kVec; idx += kThr) {  // T upper triangular
       const int i = idx / kVec, k = idx % kVec;
       double2 s = make_double2(0, 0);
-      for (int q = i; q < kNB; ++q) cfma(s, T[i * 17 + q], W[q * kLdz + k]);
+      if (ADJ)
+        for (int q = 0; q <= i; ++q) cfmac(s, T[q * 17 + i], W[q * kLdz + k]);
+      else
+        for (int q = i; q < kNB; ++q) cfma(s, T[i * 17 + q], W[q * kLdz + k]);
       W2[i * kLdz + k] = s;
     }
     __syncthreads();
@@ -1267,15 +1284,74 @@ __global__ void __launch_bounds__(kThr, 2) panel_back_kernel(const EigItem* __re
   }
 }
 
-template <int NB>
+template <int NB, bool ADJ>
 cudaError_t launch_panel_back(const EigItem* items, int nitems, int ld, int max_nvec, const double2* hbuf,
                               double2* zbuf, const int* info, cudaStream_t st) {
   const size_t sm = panel_back_smem<NB>(ld);
   const cudaError_t e =
-      cudaFuncSetAttribute(panel_back_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaFuncSetAttribute(panel_back_kernel<NB, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  panel_back_kernel<NB><<<dim3(nitems, (max_nvec + 8 * NB - 1) / (8 * NB)), kThr, sm, st>>>(items, hbuf, zbuf, info);
+  panel_back_kernel<NB, ADJ><<<dim3(nitems, (max_nvec + 8 * NB - 1) / (8 * NB)), kThr, sm, st>>>(items, hbuf, zbuf,
+                                                                                              info);
   return cudaGetLastError();
+}
+
+// Q (or Q^H) on the vectors of every item
+template <bool ADJ>
+cudaError_t apply_q(const EigItem* items, int nitems, int ld, int max_nvec, const double2* hbuf, const double2* rbuf,
+                    double2* zbuf, const int* info, cudaStream_t st) {
+  constexpr int kVec = 32 / kBackLanes;
+  const auto band = [&]() {
+    band_back_kernel<ADJ><<<dim3(nitems, (max_nvec + kVec - 1) / kVec), 32, 0, st>>>(items, rbuf, zbuf, info);
+    return cudaGetLastError();
+  };
+  // 16 vectors a CTA while two CTAs share an SM (ld <= 304), else 8
+  const auto panels = [&]() {
+    return max_nvec > 8 && panel_back_smem<2>(ld) <= 112 * 1024
+               ? launch_panel_back<2, ADJ>(items, nitems, ld, max_nvec, hbuf, zbuf, info, st)
+               : launch_panel_back<1, ADJ>(items, nitems, ld, max_nvec, hbuf, zbuf, info, st);
+  };
+  const cudaError_t e = ADJ ? panels() : band();
+  return e != cudaSuccess ? e : (ADJ ? band() : panels());
+}
+
+// x <- -(T - lam_k)^-1 x for the complex vectors of every item, in place; eigenvalue
+// lam_k of item b at lam[w_off + k]. Two threads per vector (real and imaginary
+// part) share one factorisation.
+constexpr int kShiftThr = 128;
+__global__ void __launch_bounds__(kShiftThr) tri_shift_kernel(const EigItem* __restrict__ items,
+                                                         const double2* __restrict__ rbuf,
+                                                         const double* __restrict__ lam, double2* __restrict__ zbuf,
+                                                         double* __restrict__ scratch) {
+  const EigItem it = items[blockIdx.x];
+  const int n = it.n, nvec = it.nev, tid = threadIdx.x;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double* d = reinterpret_cast<double*>(smraw);
+  double* e = d + n;
+  __shared__ double red[kShiftThr / 32];
+  load_tri(it, rbuf, d, e);
+  double tn = 0.0;
+  for (int i = tid; i < n; i += kShiftThr)
+    tn = fmax(tn, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
+  if ((tid & 31) == 0) red[tid >> 5] = tn;
+  __syncthreads();
+  tn = fmax(fmax(red[0], red[1]), fmax(red[2], red[3]));
+  for (int i = tid; i < n - 1; i += kShiftThr)
+    if (fabs(e[i]) <= DBL_EPSILON * (fabs(d[i]) + fabs(d[i + 1]))) e[i] = 0.0;
+  __syncthreads();
+  const double tiny = fmax(DBL_EPSILON * tn, 1e-290);
+  const int ldv = tri_ldv(nvec);
+  double* F = scratch + it.s_off;
+  double* I0 = F + (size_t)n * ldv;
+  for (int k = tid; k < nvec; k += kShiftThr) tri_factor(d, e, n, lam[it.w_off + k], tiny, F + k, I0 + k, ldv);
+  __syncthreads();
+  for (int x = tid; x < 2 * nvec; x += kShiftThr) {
+    const int k = x >> 1;
+    double* xb = reinterpret_cast<double*>(zbuf + it.z_off + (size_t)k * n) + (x & 1);
+    tri_factored_solve(d, e, lam[it.w_off + k], F + k, I0 + k, ldv, n, xb, 2, -1.0);
+  }
 }
 
 // ------------------------------------------------------------------- host
@@ -1322,14 +1398,22 @@ cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nv
   }
   e = cudaGetLastError();
   if (max_nvec > 0 && e == cudaSuccess) {
-    constexpr int kVec = 32 / kBackLanes;
-    band_back_kernel<<<dim3(nitems, (max_nvec + kVec - 1) / kVec), 32, 0, st>>>(items, rbuf, zbuf, info);
-    // 16 vectors a CTA while two CTAs share an SM (ld <= 304), else 8
-    e = max_nvec > 8 && panel_back_smem<2>(ld) <= 112 * 1024
-            ? launch_panel_back<2>(items, nitems, ld, max_nvec, hbuf, zbuf, info, st)
-            : launch_panel_back<1>(items, nitems, ld, max_nvec, hbuf, zbuf, info, st);
+    e = apply_q<false>(items, nitems, ld, max_nvec, hbuf, rbuf, zbuf, info, st);
   }
   return e;
+}
+
+cudaError_t launch_heev2_resolvent(const EigItem* items, int nitems, int max_n, int max_nvec, const double2* hbuf,
+                                   const double2* rbuf, const double* lam, double2* zbuf, double* scratch,
+                                   const int* info, cudaStream_t st) {
+  if (nitems <= 0 || max_nvec <= 0) return cudaSuccess;
+  const int ld = heev2_ld(max_n);
+  cudaError_t e = apply_q<true>(items, nitems, ld, max_nvec, hbuf, rbuf, zbuf, info, st);
+  if (e != cudaSuccess) return e;
+  tri_shift_kernel<<<nitems, kShiftThr, sizeof(double) * 2 * max_n, st>>>(items, rbuf, lam, zbuf, scratch);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return apply_q<false>(items, nitems, ld, max_nvec, hbuf, rbuf, zbuf, info, st);
 }
 
 }  // namespace dev

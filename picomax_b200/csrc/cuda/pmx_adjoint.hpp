@@ -96,6 +96,9 @@ struct ResolventArgs {
   double* work;         // [item][8][5 n] doubles
 };
 cudaError_t launch_resolvent(const ResolventArgs& a, cudaStream_t st);
+// out = a - b, and y += a - b (count complex values)
+cudaError_t launch_sub(const double2* a, const double2* b, double2* out, long long count, cudaStream_t st);
+cudaError_t launch_add_sub(const double2* a, const double2* b, double2* y, long long count, cudaStream_t st);
 
 // X = diag(lbar) Z (Hellmann-Feynman only): X [batch][ns][n], Z stride zs.
 cudaError_t launch_hf_x(const double2* Z, long long zs, const double* lbar, int n, int ns, int batch, double2* X,

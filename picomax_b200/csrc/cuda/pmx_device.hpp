@@ -88,6 +88,13 @@ bool heev2_supported(int max_n);
 size_t heev2_rbuf_double2(int ld, int launch_ld);
 cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nval, int max_nvec, double2* hbuf,
                          double* wbuf, double2* zbuf, double* scratch, double2* rbuf, int* info, cudaStream_t st);
+// After launch_heev2, with its reduction H = Q T Q^H still in hbuf and rbuf:
+// x <- Q (lam_k - T)^-1 Q^H x for vectors k < nev of every item (z_off in zbuf),
+// eigenvalue lam_k at lam[w_off + k]; scratch: 4 n nev doubles at s_off. The caller
+// projects out the eigenvectors that make lam_k - T singular.
+cudaError_t launch_heev2_resolvent(const EigItem* items, int nitems, int max_n, int max_nvec, const double2* hbuf,
+                                   const double2* rbuf, const double* lam, double2* zbuf, double* scratch,
+                                   const int* info, cudaStream_t st);
 
 // Symmetry reduction of a Gamma-centred n[0] x n[1] x n[2] grid (kgrid.cu):
 // ops are integer matrices in the reciprocal basis (a group, identity

@@ -271,11 +271,11 @@ __device__ inline void tri_factor(const double* __restrict__ d, const double* __
 __device__ __forceinline__ bool tri_swapped(double f) { return (__double_as_longlong(f) & 1ll) != 0; }
 
 // Solves (T - lam I) x = scale b in place with the factors of tri_factor: x (b on
-// entry) at xb[i * st]; returns |x|^2. Division-free; the loads of eight rows run
+// entry) at xb[i * xs]; returns |x|^2. Division-free; the loads of eight rows run
 // ahead of the recurrences (the next eight while these are worked on).
 __device__ inline double tri_factored_solve(const double* __restrict__ d, const double* __restrict__ e, double lam,
                                             const double* __restrict__ F, const double* __restrict__ I0, int st, int n,
-                                            double* __restrict__ xb, double scale) {
+                                            double* __restrict__ xb, int xs, double scale) {
   constexpr int kB = 8;
   double xc = scale * xb[0];
   {
@@ -284,7 +284,7 @@ __device__ inline double tri_factored_solve(const double* __restrict__ d, const 
 #pragma unroll
       for (int u = 0; u < kB; ++u) {
         const int i = i0 + u;
-        x[u] = i + 1 < n ? xb[(size_t)(i + 1) * st] : 0.0;
+        x[u] = i + 1 < n ? xb[(size_t)(i + 1) * xs] : 0.0;
         f[u] = i + 1 < n ? F[(size_t)i * st] : 0.0;
       }
     };
@@ -298,7 +298,7 @@ __device__ inline double tri_factored_solve(const double* __restrict__ d, const 
           const double xi = scale * xv[u];
           const bool sw = tri_swapped(fv[u]);
           const double piv = sw ? xi : xc, oth = sw ? xc : xi;
-          xb[(size_t)i * st] = piv;
+          xb[(size_t)i * xs] = piv;
           xc = fma(-fv[u], piv, oth);
         }
         xv[u] = xn[u];
@@ -307,14 +307,14 @@ __device__ inline double tri_factored_solve(const double* __restrict__ d, const 
     }
   }
   double x1 = xc * I0[(size_t)(n - 1) * st], x2 = 0.0;  // rows i + 1, i + 2
-  xb[(size_t)(n - 1) * st] = x1;
+  xb[(size_t)(n - 1) * xs] = x1;
   double s = x1 * x1;
   double yv[kB], iv[kB], fv[kB], yn[kB], in[kB], fn[kB];
   auto load = [&](int i0, double (&y)[kB], double (&p)[kB], double (&f)[kB]) {
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 - u;
-      y[u] = i >= 0 ? xb[(size_t)i * st] : 0.0;
+      y[u] = i >= 0 ? xb[(size_t)i * xs] : 0.0;
       p[u] = i >= 0 ? I0[(size_t)i * st] : 0.0;
       f[u] = i >= 1 ? F[(size_t)(i - 1) * st] : 0.0;  // of the row above
     }
@@ -333,7 +333,7 @@ __device__ inline double tri_factored_solve(const double* __restrict__ d, const 
         const double c = tri_swapped(fv[u]) ? -fv[u] * e[i] : e[i];
         const double u1 = sw ? d[i + 1] - lam : c, u2 = sw && i + 1 < n - 1 ? e[i + 1] : 0.0;
         const double xi = fma(-u1, x1, fma(-u2, x2, yv[u])) * iv[u];
-        xb[(size_t)i * st] = xi;
+        xb[(size_t)i * xs] = xi;
         s = fma(xi, xi, s);
         x2 = x1;
         x1 = xi;
@@ -401,7 +401,7 @@ __device__ inline void tri_eigvecs(const TriWork& W, int n, int nvec, double2* _
   const int ncl = W.misc[0];
   for (int iter = 0; iter < kTriInvIters; ++iter) {
     for (int k = tid; k < nvec; k += nthr)
-      rn[k] = inv_norm(k, tri_factored_solve(d, e, lam[k], F + k, I0 + k, ldv, n, X + k, rn[k]));
+      rn[k] = inv_norm(k, tri_factored_solve(d, e, lam[k], F + k, I0 + k, ldv, n, X + k, ldv, rn[k]));
     __syncthreads();
     for (int cl = wid; cl < ncl; cl += nthr / 32) {
       const int c0 = W.clus[cl], c1 = W.clus[cl + 1];

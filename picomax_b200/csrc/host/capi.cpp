@@ -272,8 +272,8 @@ struct pmx_ctx {
   DevBuf t_wk, t_wq, t_kw, t_ntr, t_nblk, t_toff, t_rsrc, t_rde, t_rw, t_rf0, t_cnt, t_sum;  // device transition list
   DevBuf m32, tcerr;  // tensor-core overlaps of the mixed path and their wait status
   // adjoint workspaces
-  DevBuf a_chi, a_g, a_gx, a_kk, a_f1, a_f2, a_obar, a_debar, a_mbar, a_zbk, a_zbq, a_lbk, a_lbq;
-  DevBuf a_lamk, a_lamq, a_C, a_X, a_R, a_SV, a_SSO, a_kp, a_linv, a_tri, a_work;
+  DevBuf a_chi, a_g, a_gx, a_kk, a_f1, a_f2, a_obar, a_debar, a_mbar, a_zb, a_lb;
+  DevBuf a_lam, a_C, a_X, a_R, a_SV, a_SSO, a_kp, a_linv, a_tri, a_work;
   // several crystals at once (batched entry points)
   DevBuf b_g, b_hkl, b_vloc, b_vso, b_crystal;
   int kk_nf = 0;                       // grid length of the Kramers-Kronig tables in kktab (0: none)
@@ -474,12 +474,12 @@ cudaError_t eig_launch(pmx_ctx* c, const pmx::dev::EigItem* items, int nitems, i
 
 // H workspace of one chunk of eigensolves: 2 GB, or up to 8 GB where two
 // waves of 148 matrices of the largest size need more (n > 832), so that the
-// large sizes still fill the GPU; 4 GB and one matrix more with the tridiagonal
-// export, whose caller keeps 2 GB at k and k + q each and the reference point
+// large sizes still fill the GPU; 4 GB and one matrix more where the reduction is
+// kept, whose caller keeps 2 GB at k and k + q each and the reference point
 // within one chunk
-size_t h_budget(size_t hbytes_max, bool tri) {
+size_t h_budget(size_t hbytes_max, bool keep) {
   const size_t base = (size_t)2 << 30;
-  return tri ? 2 * base + hbytes_max : std::max(base, std::min((size_t)8 << 30, 296 * hbytes_max));
+  return keep ? 2 * base + hbytes_max : std::max(base, std::min((size_t)8 << 30, 296 * hbytes_max));
 }
 
 // One set of eigenproblems of a crystal: H(k) of every k, the lowest nval
@@ -496,11 +496,12 @@ struct SolveSet {
 // stages take one or two matrices per SM, so that a set of its own (above all the
 // single matrix of the reference energy) would pay for a wave of SMs it does not
 // fill. zdev may be null when no set has vectors.
-// With tri (device, [items][4 n], items in set order) the tridiagonal form of every
-// H(k) is exported and the reflectors of the last chunk stay in c->hbuf (all sets
-// must then fit one chunk, see h_budget).
+// With keep the reduction H = Q T Q^H of every item stays behind for the adjoint (all
+// sets must then fit one chunk, see h_budget): of the two-stage solver in c->hbuf and
+// c->rbuf, items in set order; below its sizes of the one-stage one, reflectors in
+// c->hbuf and the tridiagonal form in tri (device, [items][4 n]).
 void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& sets, double2* zdev,
-                double* tri = nullptr) {
+                bool keep = false, double* tri = nullptr) {
   const int n = dc.n;
   int nk = 0, nval = 0, nvec = 0;
   for (const SolveSet& s : sets) {
@@ -516,8 +517,9 @@ void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& s
   const bool tri_req = tri != nullptr;
   const int ld = eig_ld(n, n, tri_req);
   const size_t hbytes = (size_t)ld * ld * sizeof(double2);
-  int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nk, h_budget(hbytes, tri_req) / hbytes));
+  int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nk, h_budget(hbytes, keep) / hbytes));
   chunk = std::min(chunk, 4096);
+  if (keep && nk > chunk) throw CudaFail("the adjoint's block does not fit one eigensolver chunk", PMX_ERR_LIMIT);
   if (nk > chunk) {  // several chunks: each a whole number of waves of CTAs
     const int unit = pmx::dev::heev_batch_unit(n, nval);
     if (chunk >= unit) chunk = chunk / unit * unit;
@@ -571,7 +573,9 @@ void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& s
     int variant = 0;
     const int nvar = eig_variants(n, nval, tri_req);
     auto it_choice = c->heev_choice.find(key);
-    if (c->fixed_schedule >= 0) {
+    if (keep) {
+      variant = 0;  // the two-stage solver where it applies
+    } else if (c->fixed_schedule >= 0) {
       variant = std::min(c->fixed_schedule, nvar - 1);
     } else if (it_choice != c->heev_choice.end()) {
       variant = it_choice->second;
@@ -1942,9 +1946,9 @@ void hf_items(pmx_ctx* c, const DevCrystal& dc, const double2* Z, long long zs, 
               const std::vector<Vec3>& ks, int ns) {
   const int nb = (int)ks.size();
   if (nb == 0) return;
-  h2d(c, c->a_lbk, lbar.data(), sizeof(double) * lbar.size());
+  h2d(c, c->a_lb, lbar.data(), sizeof(double) * lbar.size());
   CK(c->a_X.ensure(sizeof(double2) * (size_t)nb * ns * dc.n));
-  CK(pmx::dev::launch_hf_x(Z, zs, c->a_lbk.as<double>(), dc.n, ns, nb, c->a_X.as<double2>(), c->stream));
+  CK(pmx::dev::launch_hf_x(Z, zs, c->a_lb.as<double>(), dc.n, ns, nb, c->a_X.as<double2>(), c->stream));
   c->launches += 1;
   hgrad_items(c, dc, c->a_X.as<double2>(), (long long)ns * dc.n, Z, zs, ks, ns);
 }
@@ -2091,8 +2095,10 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
     // of the rest; a block's reflectors must fit one eigensolver chunk.
     int nsx = std::min(n, ns + 8);
     // (2 kb + 1 matrices make one eigensolver chunk, at most 4096)
+    const bool two_stage = use_two_stage(n, false);
+    const int ld = eig_ld(n, n, !two_stage);
     const int kb = (int)std::max<size_t>(
-        1, std::min<size_t>({(size_t)nk, ((size_t)2 << 30) / ((size_t)n * n * 16), (size_t)2047}));
+        1, std::min<size_t>({(size_t)nk, ((size_t)2 << 30) / ((size_t)ld * ld * 16), (size_t)2047}));
     (void)nall;
     CK(ctx->a_kk.ensure(sizeof(double) * 2 * (size_t)np * nf));
     CK(ctx->chi2.ensure(sizeof(double) * 2 * (size_t)np * nf));
@@ -2138,13 +2144,13 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
           // tridiagonals and reflectors of the k side first, then of the k + q side
           const long long zs = (long long)cnt * nvs * n;
           CK(ctx->zk.ensure(sizeof(double2) * 2 * (size_t)zs));
-          CK(ctx->a_tri.ensure(sizeof(double) * 4 * (size_t)(2 * cnt + 1) * n));
+          if (!two_stage) CK(ctx->a_tri.ensure(sizeof(double) * 4 * (size_t)(2 * cnt + 1) * n));
           {
             Timer tm(ctx, 0);
             std::vector<SolveSet> sets{{ks, nvl, nvs, 0, &wk}, {kqs, nvl, nvs, zs, &wq}};
             const bool first = ref.w.empty() && !ref_set.ks.empty();
             if (first) sets.push_back(ref_set);
-            solve_sets(ctx, dc, sets, ctx->zk.as<double2>(), ctx->a_tri.as<double>());
+            solve_sets(ctx, dc, sets, ctx->zk.as<double2>(), true, two_stage ? nullptr : ctx->a_tri.as<double>());
             if (first) off = ref.energy(p, dc.soc);
           }
           // the projected prefix must not split a degenerate set
@@ -2174,14 +2180,12 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
         h2d(ctx, ctx->wgt, T.wgt.data(), sizeof(double) * T.wgt.size());
         const int ncd_max = T.ncd.empty() ? 0 : *std::max_element(T.ncd.begin(), T.ncd.end());
         const int nvd_max = T.nvd.empty() ? 0 : *std::max_element(T.nvd.begin(), T.nvd.end());
-        CK(ctx->a_zbk.ensure(sizeof(double2) * (size_t)cnt * ns * n));
-        CK(ctx->a_zbq.ensure(sizeof(double2) * (size_t)cnt * ns * n));
-        CK(cudaMemsetAsync(ctx->a_zbk.ptr, 0, sizeof(double2) * (size_t)cnt * ns * n, st));
-        CK(cudaMemsetAsync(ctx->a_zbq.ptr, 0, sizeof(double2) * (size_t)cnt * ns * n, st));
-        CK(ctx->a_lbk.ensure(sizeof(double) * (size_t)cnt * ns));
-        CK(ctx->a_lbq.ensure(sizeof(double) * (size_t)cnt * ns));
-        CK(cudaMemsetAsync(ctx->a_lbk.ptr, 0, sizeof(double) * (size_t)cnt * ns, st));
-        CK(cudaMemsetAsync(ctx->a_lbq.ptr, 0, sizeof(double) * (size_t)cnt * ns, st));
+        // dL/dz and dL/dlambda of both sides, the k side first
+        const size_t zb = (size_t)cnt * ns * n;
+        CK(ctx->a_zb.ensure(sizeof(double2) * 2 * zb));
+        CK(cudaMemsetAsync(ctx->a_zb.ptr, 0, sizeof(double2) * 2 * zb, st));
+        CK(ctx->a_lb.ensure(sizeof(double) * 2 * (size_t)cnt * ns));
+        CK(cudaMemsetAsync(ctx->a_lb.ptr, 0, sizeof(double) * 2 * (size_t)cnt * ns, st));
         if (T.T > 0) {
           const int A = 3 * neps;
           CK(ctx->M.ensure(sizeof(double2) * (size_t)T.T * A));
@@ -2284,10 +2288,10 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
           za.linv = ctx->a_linv.as<int>();
           za.mbar = ctx->a_mbar.as<double2>();
           za.dEbar = ctx->a_debar.as<double>();
-          za.zbar_k = ctx->a_zbk.as<double2>();
-          za.zbar_q = ctx->a_zbq.as<double2>();
-          za.lbar_k = ctx->a_lbk.as<double>();
-          za.lbar_q = ctx->a_lbq.as<double>();
+          za.zbar_k = ctx->a_zb.as<double2>();
+          za.zbar_q = ctx->a_zb.as<double2>() + zb;
+          za.lbar_k = ctx->a_lb.as<double>();
+          za.lbar_q = ctx->a_lb.as<double>() + (size_t)cnt * ns;
           {
             KTime kt(ctx, "adj_zbar");
             CK(pmx::dev::launch_zbar(za, st));
@@ -2296,51 +2300,81 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
         }
         // eigenproblem adjoint of both sides, then the pair accumulators
         Timer tm(ctx, 3);
-        h2d(ctx, ctx->a_lamk, wk.data(), sizeof(double) * wk.size());
-        h2d(ctx, ctx->a_lamq, wq.data(), sizeof(double) * wq.size());
-        const size_t cz = (size_t)cnt * ns * nsx;
+        const int nb = 2 * cnt;
+        std::vector<double> lamh(wk);
+        lamh.insert(lamh.end(), wq.begin(), wq.end());
+        h2d(ctx, ctx->a_lam, lamh.data(), sizeof(double) * lamh.size());
+        const size_t cz = (size_t)nb * ns * nsx;
         CK(ctx->a_C.ensure(sizeof(double2) * 2 * cz));
-        CK(ctx->a_X.ensure(sizeof(double2) * (size_t)cnt * ns * n));
-        CK(ctx->a_work.ensure(sizeof(double) * (size_t)cnt * 8 * 5 * n));
-        for (int side = 0; side < 2; ++side) {
-          const double2* Z = side == 0 ? ctx->zk.as<double2>() : (ctx->zk.as<double2>() + (long long)cnt * nvs * n);
-          const double2* Zb = side == 0 ? ctx->a_zbk.as<double2>() : ctx->a_zbq.as<double2>();
-          const double* lam = side == 0 ? ctx->a_lamk.as<double>() : ctx->a_lamq.as<double>();
-          const double* lb = side == 0 ? ctx->a_lbk.as<double>() : ctx->a_lbq.as<double>();
-          double2* C = ctx->a_C.as<double2>();
-          {
-            KTime kt(ctx, "adj_eig");
-            // X = Z_S' K (prefix part) ...
-            CK(pmx::dev::launch_zgemm_batched(1, nsx, ns, n, Z, n, (long long)nvs * n, Zb, n, (long long)ns * n, C,
-                                              nsx, (long long)ns * nsx, cnt, st));
-            CK(pmx::dev::launch_eig_kmat(C, lam, nvl, lb, nsx, ns, cnt, tau, st));
-            CK(pmx::dev::launch_zgemm_batched(0, n, ns, nsx, Z, n, (long long)nvs * n, C + cz, nsx,
-                                              (long long)ns * nsx, ctx->a_X.as<double2>(), n, (long long)ns * n, cnt,
-                                              st));
-          }
-          {
-            // ... + P (lam_k - H)^-1 P zbar_k for the rest of the spectrum
-            KTime kt(ctx, "adj_resolvent");
-            pmx::dev::ResolventArgs ra{};
-            ra.n = n;
-            ra.ns = ns;
-            ra.nsx = nsx;
-            ra.nitems = cnt;
-            ra.H = ctx->hbuf.as<double2>() + (side == 0 ? 0 : (size_t)cnt * n * n);
-            ra.tri = ctx->a_tri.as<double>() + (side == 0 ? 0 : (size_t)4 * cnt * n);
-            ra.lam = lam;
-            ra.lam_stride = nvl;
-            ra.Z = Z;
-            ra.zs = (long long)nvs * n;
-            ra.zbar = Zb;
-            ra.Y = ctx->a_X.as<double2>();
-            ra.work = ctx->a_work.as<double>();
-            CK(pmx::dev::launch_resolvent(ra, st));
-          }
-          ctx->launches += 4;
-          hgrad_items(ctx, dc, ctx->a_X.as<double2>(), (long long)ns * n, Z, (long long)nvs * n,
-                      side == 0 ? ks : kqs, ns);
+        CK(ctx->a_X.ensure(sizeof(double2) * 2 * zb));
+        const double2* Z = ctx->zk.as<double2>();
+        const double2* Zb = ctx->a_zb.as<double2>();
+        const double* lam = ctx->a_lam.as<double>();
+        double2* C = ctx->a_C.as<double2>();
+        double2* X = ctx->a_X.as<double2>();
+        const long long zs = (long long)nvs * n, ys = (long long)ns * n, cs = (long long)ns * nsx;
+        {
+          KTime kt(ctx, "adj_eig");
+          // X = Z_S' K (prefix part) ...
+          CK(pmx::dev::launch_zgemm_batched(1, nsx, ns, n, Z, n, zs, Zb, n, ys, C, nsx, cs, nb, st));
+          CK(pmx::dev::launch_eig_kmat(C, lam, nvl, ctx->a_lb.as<double>(), nsx, ns, nb, tau, st));
+          CK(pmx::dev::launch_zgemm_batched(0, n, ns, nsx, Z, n, zs, C + cz, nsx, cs, X, n, ys, nb, st));
         }
+        if (two_stage) {
+          // ... + P (lam_k - H)^-1 P zbar_k for the rest of the spectrum, with Q of the
+          // two-stage reduction and P = 1 - Z_S' Z_S'^H
+          KTime kt(ctx, "adj_resolvent");
+          CK(ctx->a_work.ensure(sizeof(double2) * 4 * zb));
+          double2* Y = ctx->a_work.as<double2>();
+          double2* PZ = Y + 2 * zb;
+          CK(pmx::dev::launch_zgemm_batched(0, n, ns, nsx, Z, n, zs, C, nsx, cs, PZ, n, ys, nb, st));
+          CK(pmx::dev::launch_sub(Zb, PZ, Y, (long long)(2 * zb), st));
+          const size_t sstride = pmx::dev::heev_scratch_doubles(n, nvs, n);
+          std::vector<pmx::dev::EigItem> items(nb);
+          for (int i = 0; i < nb; ++i) {
+            pmx::dev::EigItem& it = items[i];
+            it = pmx::dev::EigItem{};
+            it.n = n;
+            it.ld = ld;
+            it.nev = ns;
+            it.want_vec = 1;
+            it.h_off = (long long)i * ld * ld;
+            it.r_off = (long long)i * (long long)eig_rstride(n, n, false);
+            it.z_off = (long long)i * ys;
+            it.w_off = (long long)i * nvl;
+            it.s_off = (long long)i * (long long)sstride;
+          }
+          h2d(ctx, ctx->items, items.data(), sizeof(pmx::dev::EigItem) * nb);
+          CK(pmx::dev::launch_heev2_resolvent(ctx->items.as<pmx::dev::EigItem>(), nb, n, ns, ctx->hbuf.as<double2>(),
+                                              ctx->rbuf.as<double2>(), lam, Y, ctx->scratch.as<double>(),
+                                              ctx->info.as<int>(), st));
+          CK(pmx::dev::launch_zgemm_batched(1, nsx, ns, n, Z, n, zs, Y, n, ys, C, nsx, cs, nb, st));
+          CK(pmx::dev::launch_zgemm_batched(0, n, ns, nsx, Z, n, zs, C, nsx, cs, PZ, n, ys, nb, st));
+          CK(pmx::dev::launch_add_sub(Y, PZ, X, (long long)(2 * zb), st));
+          ctx->launches += 13;
+        } else {
+          KTime kt(ctx, "adj_resolvent");
+          CK(ctx->a_work.ensure(sizeof(double) * (size_t)nb * 8 * 5 * n));
+          pmx::dev::ResolventArgs ra{};
+          ra.n = n;
+          ra.ns = ns;
+          ra.nsx = nsx;
+          ra.nitems = nb;
+          ra.H = ctx->hbuf.as<double2>();
+          ra.tri = ctx->a_tri.as<double>();
+          ra.lam = lam;
+          ra.lam_stride = nvl;
+          ra.Z = Z;
+          ra.zs = zs;
+          ra.zbar = Zb;
+          ra.Y = X;
+          ra.work = ctx->a_work.as<double>();
+          CK(pmx::dev::launch_resolvent(ra, st));
+          ctx->launches += 4;
+        }
+        std::vector<Vec3> kall(ks);
+        kall.insert(kall.end(), kqs.begin(), kqs.end());
+        hgrad_items(ctx, dc, X, ys, Z, zs, kall, ns);
       }
     }
     adj_finish(ctx, P, dc, grad);
