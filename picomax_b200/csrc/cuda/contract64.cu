@@ -183,15 +183,19 @@ __global__ void __launch_bounds__(kThr, 2) contract64_kernel(ContractArgs a, con
     const int b = idx / ((kRows - 2 * kPairs) * kPLd), r = idx % ((kRows - 2 * kPairs) * kPLd);
     sP[b * kRows * kPLd + 2 * kPairs * kPLd + r] = 0.0;
   }
+  // overlap e of the block is always copied by the same threads, kTPh transitions apart
+  constexpr int kTPh = kThr / kElems;
+  const int se = tid % kElems, st0 = tid / kElems;
+  const int side = se / (kAB * NCH), sr = se - side * (kAB * NCH), sab = (side ? b0 : a0) + sr / NCH;
+  const double2* ssrc = a.M + (size_t)min(sab, A - 1) * NCH + sr % NCH;
   auto stage_m = [&](int buf, int t0) {
-    double2* dst = sM + buf * kElems * kTK;
-    for (int idx = tid; idx < kElems * kTK; idx += kThr) {
-      const int t = idx / kElems, e = idx - t * kElems;
-      const int side = e / (kAB * NCH), r = e - side * (kAB * NCH);
-      const int ab = (side ? b0 : a0) + r / NCH;
-      const bool ok = t0 + t < tr.y && ab < A;
-      const double2* src = a.M + (ok ? ((size_t)(t0 + t) * A + ab) * NCH + r % NCH : 0);
-      cp_async16_zfill(dst + midx(e, t), src, ok);
+    if (st0 < kTPh) {
+      double2* dst = sM + buf * kElems * kTK;
+#pragma unroll
+      for (int t = st0; t < kTK; t += kTPh) {
+        const bool ok = t0 + t < tr.y && sab < A;
+        cp_async16_zfill(dst + midx(se, t), ssrc + (size_t)(ok ? t0 + t : 0) * A * NCH, ok);
+      }
     }
     cp_async_commit();
   };
