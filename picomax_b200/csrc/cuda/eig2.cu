@@ -59,6 +59,7 @@ constexpr int kThr = 256;      // threads per CTA of every stage
 constexpr int kNW = kThr / 32;
 constexpr int kMaxLd = 1216;   // largest padded dimension
 constexpr int kVSmemLd = 800;  // largest one whose stage-1 V fits in shared memory
+constexpr int kSmallLd = 160;  // up to it stages 1 and 2 run two CTAs per SM
 constexpr int kSmemLd = 416;   // largest one whose stage-1 Y and stage-2 band fit in shared memory
 
 // element (r, c) of an m x 16 complex panel in shared memory: rows of 16,
@@ -508,8 +509,9 @@ __device__ __forceinline__ double2 ldy(const double2* p) {
 
 // KYG: Y in the item's work area of the reflector buffer (ld > kSmemLd);
 // KVG: V there too (ld > kVSmemLd)
-template <int MR, bool KYG, bool KVG = false>
-__global__ void __launch_bounds__(kThr, 1) sb_kernel(const EigItem* __restrict__ items, double2* __restrict__ hbuf,
+// OCC: CTAs per SM
+template <int MR, bool KYG, bool KVG = false, int OCC = 1>
+__global__ void __launch_bounds__(kThr, OCC) sb_kernel(const EigItem* __restrict__ items, double2* __restrict__ hbuf,
                                                     double2* __restrict__ rbuf) {
   const EigItem it = items[blockIdx.x];
   const int ld = it.ld;
@@ -659,9 +661,7 @@ __global__ void __launch_bounds__(kThr, 1) sb_kernel(const EigItem* __restrict__
 // tasks of the sweep before, with a barrier per step and checks of every row and
 // column (1770 warp instructions a task, now 1000 with the polls).
 constexpr int kBandLd = 2 * kNB;
-constexpr int kPairs = 8;                // sweeps in flight: one per pair of warps
-constexpr int kS2Thr = 64 * kPairs;      // a D warp and an E warp per pair
-constexpr int kS2W = kS2Thr / 32;
+constexpr int kMaxPairs = 8;             // sweeps in flight: one per pair of warps (a D and an E warp)
 constexpr int kProgStride = 128;         // progress word: sweep * 128 + half steps done
 // a reflector slot: entries 0..7 at 0, 8..15 at 9 (the two halves of a warp read
 // them from different banks), tau at 17
@@ -670,8 +670,8 @@ __device__ __forceinline__ int vidx(int r) { return r + (r >> 3); }
 constexpr long long kWaitNs = 2000000000LL;  // default limit of one wait
 
 __host__ __device__ inline size_t band_double2(int ld) { return (size_t)(ld + kNB) * kBandLd; }
-__host__ __device__ inline size_t sbtrd_smem_bytes(int ld, bool bg) {
-  return sizeof(double2) * ((bg ? 0 : band_double2(ld)) + kPairs * 2 * kSlot + kS2W * kSlot) + sizeof(int) * (2 * kPairs + 4);
+__host__ __device__ inline size_t sbtrd_smem_bytes(int ld, int pairs, bool bg) {
+  return sizeof(double2) * ((bg ? 0 : band_double2(ld)) + pairs * 4 * kSlot) + sizeof(int) * (2 * pairs + 4);
 }
 
 __device__ __forceinline__ int ld_acquire_shared(const int* p) {
@@ -733,9 +733,10 @@ __device__ __forceinline__ void add_halves(double2& v) {
 // KBG: the band in the item's work area of the reflector buffer (ld >
 // kSmemLd; a CTA-private region, so the same CTA-scope ordering as in shared
 // memory applies)
-template <bool KBG>
-__global__ void __launch_bounds__(kS2Thr, 1) sbtrd_kernel(const EigItem* __restrict__ items,
+template <int kPairs, bool KBG>
+__global__ void __launch_bounds__(64 * kPairs, kMaxPairs / kPairs) sbtrd_kernel(const EigItem* __restrict__ items,
                                                         const double2* __restrict__ hbuf, double2* __restrict__ rbuf) {
+  constexpr int kS2Thr = 64 * kPairs, kS2W = kS2Thr / 32;
   const EigItem it = items[blockIdx.x];
   const int ld = it.ld;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1372,7 +1373,9 @@ cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nv
   const int mr = sb_rows(ld);
   const bool big = ld > kSmemLd;  // Y and the band in the reflector buffer's work areas
   const size_t s1 = sb_smem_bytes(ld, mr, big, ld > kVSmemLd);
-  auto sb = mr == 9    ? sb_kernel<9, false>
+  // up to kSmallLd two CTAs per SM, although 128 registers spill a little, once there
+  // are more matrices than SMs
+  auto sb = mr == 9    ? (nitems > 148 ? sb_kernel<9, false, false, 2> : sb_kernel<9, false>)
             : mr == 17 ? sb_kernel<17, false>
             : mr == 25 ? sb_kernel<25, false>
             : mr == 36 ? sb_kernel<36, true>
@@ -1381,11 +1384,16 @@ cudaError_t launch_heev2(const EigItem* items, int nitems, int max_n, int max_nv
   e = cudaFuncSetAttribute(sb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
   if (e != cudaSuccess) return e;
   sb<<<nitems, kThr, s1, st>>>(items, hbuf, rbuf);
-  const size_t s2 = sbtrd_smem_bytes(ld, big);
-  auto tr = big ? sbtrd_kernel<true> : sbtrd_kernel<false>;
+  // small matrices have at most ten steps a sweep, which four pairs of warps keep up
+  // with: two CTAs per SM then, once there are more matrices than SMs
+  // (measured with both: 1025 matrices of n = 113 3.89 -> 3.17 ms, 433 1.77 -> 1.57;
+  // 122 with one CTA per SM 0.71, with the two-CTA kernels 0.77)
+  const int pairs = ld <= kSmallLd && nitems > 148 ? 4 : kMaxPairs;
+  const size_t s2 = sbtrd_smem_bytes(ld, pairs, big);
+  auto tr = big ? sbtrd_kernel<8, true> : (pairs == 4 ? sbtrd_kernel<4, false> : sbtrd_kernel<8, false>);
   e = cudaFuncSetAttribute(tr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
   if (e != cudaSuccess) return e;
-  tr<<<nitems, kS2Thr, s2, st>>>(items, hbuf, rbuf);
+  tr<<<nitems, 64 * pairs, s2, st>>>(items, hbuf, rbuf);
   const size_t s3 = tri_smem_bytes(max_n, max_nval);
   e = cudaFuncSetAttribute(tri_val_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
   if (e != cudaSuccess) return e;

@@ -42,3 +42,18 @@ def test_two_stage_edges(ctx, n, nev, kind):
         R = A[b] @ Z[b] - Z[b] * w[b]
         assert np.max(np.linalg.norm(R, axis=0)) < 1e-10 * scale
         assert np.max(np.abs(Z[b].conj().T @ Z[b] - np.eye(nev))) < 1e-10
+
+
+@pytest.mark.parametrize("n,nev", [(96, 8), (113, 9), (129, 16), (160, 5)])
+def test_many_small_matrices(ctx, n, nev):
+    """More small matrices than SMs: two CTAs per SM in both reduction stages."""
+    rng = np.random.default_rng(n)
+    A = np.stack([_matrix(rng, n, ("dense", "banded", "blocks", "diagonal")[b % 4]) for b in range(151)])
+    w, Z = ctx.heev(A, nev)
+    for b in (0, 1, 2, 3, 75, 147, 148, 149, 150):
+        full = np.linalg.eigvalsh(A[b])
+        scale = max(np.max(np.abs(full)), 1.0)
+        assert np.max(np.abs(w[b] - full[:nev])) < 1e-12 * scale * n
+        R = A[b] @ Z[b] - Z[b] * w[b]
+        assert np.max(np.linalg.norm(R, axis=0)) < 1e-10 * scale
+        assert np.max(np.abs(Z[b].conj().T @ Z[b] - np.eye(nev))) < 1e-10
