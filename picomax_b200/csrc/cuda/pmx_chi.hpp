@@ -100,6 +100,7 @@ struct ContractArgs {
   const int2* trange;   // [n f-tiles] transition range of each frequency tile
   int neps, np, nf, nch;
   int window;           // half width, or -1 for all frequencies
+  int zeros;            // the window only leaves out zeros of the line shape
   int delta;            // broadening model
   double eps, dfreq;
   double* acc;          // [2][9][np][nf] Re then Im
