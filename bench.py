@@ -400,7 +400,7 @@ def heev_roofline(m, fp64_peak=None):
     ach = flops / nl / (ms_launch * 1e-3) / 1e12
     bpm = profiled_heev_bytes(n)
     pk = fp64_peak or FP64_TFLOPS_NOMINAL
-    return {"kernel": "heev (two-stage: sb_kernel, sbtrd_kernel, tri_eig_kernel, eig2_back_kernel)",
+    return {"kernel": "heev (two-stage: sb_kernel, sbtrd_kernel, tri_val/vec_kernel, band_back_kernel, panel_back_kernel)",
             "bound": "fp64", "achieved": ach, "peak": pk, "unit": "TFLOP/s",
             "frac": ach / pk, "frac_of_nominal": ach / FP64_TFLOPS_NOMINAL,
             "traffic": bpm * m["nsolves"] / nl if bpm else None,

@@ -20,8 +20,8 @@
 // launch where three blocks or more share it and the table stays within 4 GB.
 // Measured on a B200 against 12 x 12 FMA tiles that also ran over the frequencies
 // where epsLL's line shape is zero: GaAs + spin-orbit epsij (216 k, 27 vectors,
-// 2000 frequencies) 18.2 -> 4.5 ms, wurtzite epsLL (144 k, 59 vectors) 249.7 ->
-// 27.6 ms, silicon epsLL (512 k, 15 vectors) 7.70 -> 0.90 ms (without the table 6.1,
+// 2000 frequencies) 18.2 -> 4.36 ms, wurtzite epsLL (144 k, 59 vectors) 249.7 ->
+// 26.9 ms, silicon epsLL (512 k, 15 vectors) 7.70 -> 0.87 ms (without the table 6.1,
 // 38.1, 1.20 ms); 16.6 and 22 TFLOP/s in the window on the first two (DGEMM 35.5).
 #include <algorithm>
 #include <cfloat>
