@@ -25,9 +25,10 @@
 // w_s^2 - w_f^2, 3.7e-14).
 //
 // Re and Im of a row are scaled by powers of two to the same size before they share
-// a sequence, and a row that is zero stays exactly zero in the other's sum. Rows
-// with non-finite or huge entries, which a transform would spread over the row, take
-// the direct sum.
+// a sequence, and a row that is zero stays exactly zero in the other's sum; entry 0,
+// which the forward transform does not weigh, has no part in that size. Rows with
+// non-finite or (but for entry 0) huge entries, which a transform would spread over
+// the row, take the direct sum.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -234,15 +235,21 @@ __global__ void __launch_bounds__(kMaxThr, 3) kk_fft_kernel(const double* __rest
   const size_t o = (size_t)blockIdx.x * nf, blk = (size_t)rows * nf;
   const double* re = in + o;
   const double* im = in + blk + o;
-  // entry 0 of the input has no weight (w_0 = 0) in the forward transform
+  // entry 0 of the input has no weight (w_0 = 0) in the forward transform: it stays out
+  // of the sequence and of the sizes that scale it (a NaN or Inf there still spreads)
   double mr = 0.0, mi = 0.0;
   int bad = 0;
   for (int s = threadIdx.x; s < nf; s += blockDim.x) {
     const double a = re[s], b = im[s];
+    if (!TR && s == 0) {
+      bad |= !isfinite(a) | !isfinite(b);
+      z[0] = make_double2(0, 0);
+      continue;
+    }
     bad |= !(fabs(a) <= 1e290) | !(fabs(b) <= 1e290);
     mr = fmax(mr, fabs(a));
     mi = fmax(mi, fabs(b));
-    z[pad(s)] = !TR && s == 0 ? make_double2(0, 0) : make_double2(a, b);
+    z[pad(s)] = make_double2(a, b);
   }
   for (int s = nf + threadIdx.x; s < l; s += blockDim.x) z[pad(s)] = make_double2(0, 0);
   bad = __syncthreads_or(bad);
