@@ -265,7 +265,8 @@ int pmx_chi_epsm(pmx_ctx* ctx, const pmx_problem* p, int sw, int precision, doub
  * (L, L) block of a chi .dat laid out [q][m][n<=m][f] (re and im arrays);
  * epsm [nq][nfreq][2]. Restates the reference's post-processing
  * include/matlab_wrapper/+picomax/+eps/macroscopic.m:13-29, :79 (MATLAB; the
- * C++ reference has no counterpart). neps <= 64. */
+ * C++ reference has no counterpart). Where [eps^-1]_00 is exactly zero (a pole
+ * of eps_M) epsm is (+inf, 0), whose loss function is zero. neps <= 64. */
 int pmx_eps_macroscopic(pmx_ctx* ctx, int neps, int nq, int nfreq, const double* chi_re, const double* chi_im,
                         double* epsm);
 

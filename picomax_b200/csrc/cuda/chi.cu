@@ -498,11 +498,15 @@ namespace dev {
 // ------------------------------------------------------------ macroscopic eps
 // eps_M(q, w) = 1 / [eps^-1]_00 with eps_mn = delta_mn + chi^LL_mn and the
 // n > m half filled by conj(eps_nm), as in the reference's post-processing
-// (include/matlab_wrapper/+picomax/+eps/macroscopic.m:13-29, :79). 1 / [eps^-1]_00
-// is the Schur complement of eps[1:, 1:]: with vector 0 last, Gaussian elimination
-// with partial pivoting among the other rows leaves it in the last diagonal
-// element, and no back substitution is needed. One CTA per (q, w), the matrix in
-// shared memory, lanes over columns and warps over rows: bound by the latency of
+// (include/matlab_wrapper/+picomax/+eps/macroscopic.m:13-29, :79). With vector 0
+// last, Gaussian elimination of eps x = e_0 with partial pivoting ends in
+// u x_0 = y, so that eps_M = 1 / x_0 = u / y without a back substitution; y is 1
+// (u is the Schur complement of eps[1:, 1:]) until row 0 itself becomes a pivot,
+// which it must where eps[1:, 1:] is near-singular (a pole of eps_M, at which the
+// loss function is regular; at the pole itself y = 0 and eps_M is infinite). From
+// then on the right-hand side is one more column, kept where that pivot's column
+// was. One CTA per (q, w), the matrix in shared memory, lanes over columns and
+// warps over rows: bound by the latency of
 // the n steps, so that several CTAs share an SM (four of 59 vectors; four warps of
 // one CTA had a matrix each before, with a serial back substitution). Measured on a
 // B200, 2000 frequencies: 59 vectors 2.06 -> 0.58 ms, 27 vectors 0.138 -> 0.089 ms, 15
@@ -525,11 +529,12 @@ __global__ void __launch_bounds__(128) epsm_kernel(const double* __restrict__ re
       if (r != c) E[ci * n + ri] = cconj(v);  // eps_nm = conj(eps_mn) above the diagonal
     }
   __syncthreads();
+  int rhs = -1;  // column of the right-hand side, once row 0 (the last row) has been a pivot
   for (int k = 0; k < n - 1; ++k) {
-    // pivot among rows k .. n - 2, the same search in every warp
+    // pivot among rows k .. n - 1, the same search in every warp
     double best = -1.0;
     int bi = k;
-    for (int r = k + lane; r < n - 1; r += 32) {
+    for (int r = k + lane; r < n; r += 32) {
       const double2 v = E[r * n + k];
       const double a = v.x * v.x + v.y * v.y;
       if (a > best) {
@@ -548,23 +553,47 @@ __global__ void __launch_bounds__(128) epsm_kernel(const double* __restrict__ re
     }
     if (bi != k) {
       __syncthreads();  // every warp has searched
-      for (int c = k + threadIdx.x; c < n; c += blockDim.x) {
-        const double2 t = E[k * n + c];
-        E[k * n + c] = E[bi * n + c];
-        E[bi * n + c] = t;
+      for (int c = k + threadIdx.x; c <= n; c += blockDim.x) {
+        const int cc = c < n ? c : rhs;
+        if (cc < 0) continue;
+        const double2 t = E[k * n + cc];
+        E[k * n + cc] = E[bi * n + cc];
+        E[bi * n + cc] = t;
       }
       __syncthreads();
     }
+    const bool row0 = rhs < 0 && bi == n - 1;  // row 0 with its right-hand side 1, the others' still 0
     const double2 p = E[k * n + k];
     const double pd = p.x * p.x + p.y * p.y;
     const double2 inv = make_double2(p.x / pd, -p.y / pd);
     for (int r = k + 1 + wid; r < n; r += nw) {
       const double2 fct = cmul(E[r * n + k], inv);
       for (int c = k + 1 + lane; c < n; c += 32) E[r * n + c] = csub(E[r * n + c], cmul(fct, E[k * n + c]));
+      if (rhs >= 0 && lane == 0) E[r * n + rhs] = csub(E[r * n + rhs], cmul(fct, E[k * n + rhs]));
+      if (row0) {
+        __syncwarp();  // the lanes have read the factor from there
+        if (lane == 0) E[r * n + k] = make_double2(-fct.x, -fct.y);
+      }
     }
+    if (row0) rhs = k;
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[job] = E[n * n - 1];
+  if (threadIdx.x == 0) {
+    double2 u = E[n * n - 1];
+    if (rhs >= 0) {
+      const double2 y = E[(n - 1) * n + rhs];
+      const double m = fmax(fabs(y.x), fabs(y.y));
+      if (y.x == 0.0 && y.y == 0.0 && (u.x != 0.0 || u.y != 0.0)) {
+        u = make_double2(INFINITY, 0.0);
+      } else {
+        const double2 ys = make_double2(y.x / m, y.y / m);
+        const double d = m * (ys.x * ys.x + ys.y * ys.y);
+        u = cmulc(ys, u);
+        u = make_double2(u.x / d, u.y / d);
+      }
+    }
+    out[job] = u;
+  }
 }
 
 cudaError_t launch_epsm(const double* re, const double* im, int neps, int nq, int nf, double2* out, cudaStream_t st) {
