@@ -10,9 +10,29 @@
 // hi*hi + hi*lo + lo*hi as tcgen05.mma kind::f16 with an FP32 accumulator in
 // TMEM (products dropped: lo*lo, ~2^-16 of each term). The transition range
 // of a frequency tile is cut into pieces; each piece adds its FP32
-// accumulator into an FP64 partial tile every 64 chunks (16 with windows of
-// zero line shape), and the pieces'
+// accumulator into an FP64 partial tile after 64 chunks or fewer, and the pieces'
 // tiles are summed in FP64 in a fixed order, so results are deterministic.
+//
+// The tensor core rounds toward zero, each addition to the accumulator and (to two
+// bits more) the products that go into it, so that an FP32 sum of terms of one sign
+// comes out too small, in proportion to its number of additions. This counts where the
+// frequencies of zero line shape are left out (epsLL, epsxyz), because the terms of one
+// frequency then stand together among the sorted transitions. There
+//  - the sums of an item interleave over all of it (sum s of n takes the transitions s,
+//    s + n, ...), so that each has only a few terms of one size at any frequency, as
+//    a sum over unsorted transitions of all frequencies would;
+//  - the sums go in pairs: the second one is subtracted from the accumulator that the
+//    first one left, S1 -> S1 - S2. Neighbours in energy have nearly the same line
+//    shape, S1 and S2 are alike, and the accumulator runs over the same values downwards
+//    and loses about as much again: with F1 and F2 its values after each, the losses
+//    cancel in S1 + S2 = 2 F1 - F2.
+// 2-norm of the error of Re chi against FP64, with FP64 overlaps (sums of 64 chunks
+// over all frequencies / of 16 neighbouring ones over windows / now): wurtzite, 59
+// vectors, 9216 k 5.9e-7 / 4.5e-6 / 5.9e-7, 1152 k 2.8e-6 / 2.9e-6 / 2.8e-6 (the BF16
+// products); Te, 384 k 2.3e-6 / 2.0e-6 / 1.4e-6. Contraction of the wurtzite spectra on a
+// B200 553 / 139 / 132 ms and 62 / 16.7 / 15.9 ms (sums of 64 chunks, with a third more
+// bias, 10 % less). The windows of epsij, and line shapes that reach everywhere, keep one
+// sum after the other.
 //
 // Pipeline of one CTA (8 producer warps + 1 control warp, two shared-memory
 // stages):
@@ -51,15 +71,15 @@ constexpr int kN = 256;        // frequencies per tile
 constexpr int kKC = 32;        // transitions per chunk
 constexpr int kProducers = 256;              // warps 0-7
 constexpr int kThreads = kProducers + 32;    // + the control warp (W copies, MMA issue)
-constexpr int kFlushChunks = 64;  // chunks (2048 transitions) per FP32 accumulation before the FP64 flush
-// The same where the frequencies of zero line shape are left out (epsLL, epsxyz).
-// There the transitions of one frequency stand together (they are sorted by window),
-// not among others whose weight is zero, so that an FP32 sum of 2048 of them adds
-// more terms than one over all frequencies. 2-norm error against FP64, Te 8x8x6 k:
-// 64 chunks 5.9e-6, 32: 3.9e-6, 16: 2.0e-6, 8: 1.1e-6 (all frequencies, 64 chunks:
-// 2.3e-6). Wurtzite, 1152 k, NEPS 59: 9.2e-6 with each (the overlaps' error);
-// contraction 13.0 / 14.4 / 16.8 / 22.2 ms (all frequencies: 62.5).
-constexpr int kFlushZeros = 16;
+constexpr int kFlushChunks = 64;  // chunks (2048 transitions) per FP32 sum before the FP64 flush, at most
+constexpr int kFlushZeros = 32;   // the same where the frequencies of zero line shape are left out
+constexpr int kMinPiece = 64;     // chunks of one CTA, at least (but for a range's last one)
+// roles of a chunk in its FP32 sum
+constexpr int kFromZero = 1;  // the accumulator starts from zero
+constexpr int kLast = 2;      // last chunk of the sum: the accumulator is flushed
+constexpr int kPair1 = 4;     // of a pair's first sum: counts twice
+constexpr int kPair2 = 8;     // of its second sum, subtracted from the first one: counts minus once
+constexpr int kStep = 16;     // from one transition of the chunk to the next, times this
 constexpr int kTargetCtas = 4 * 148;  // K-split so that the grid covers the SMs a few times
 constexpr unsigned kWaitLimit = 1u << 26;
 constexpr uint64_t kWaitNs = 2000000000ull;  // 2 s, unless the caller sets a limit
@@ -162,11 +182,8 @@ struct Plan {
   int nchunk;        // W chunks over all frequency tiles
   int nitem;         // (frequency tile, piece) items
   // device arrays inside the workspace
-  int* chunk_ft;     // [nchunk] frequency tile of the chunk
-  int* chunk_t0;     // [nchunk] first sorted transition of the chunk
-  int* chunk_t1;     // [nchunk] end of the frequency tile's range
+  int4* chunk;       // [nchunk] (frequency tile, first sorted transition, end of its item's, role + step * kStep)
   int4* item;        // [nitem] (ft, first chunk, end chunk, -)
-  int flush;         // chunks per FP64 flush
   int2* ft_items;    // [nft] (first item, end item)
   int2* tiles;       // [ntile] (a block, b block)
   float* wgt32;      // [T]
@@ -201,7 +218,8 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // -------------------------------------------------------- W chunk producer
 __global__ void __launch_bounds__(256) wgen_kernel(Plan pl, ContractArgs a) {
   const int c = blockIdx.x;
-  const int ft = pl.chunk_ft[c], t0 = pl.chunk_t0[c], t1 = pl.chunk_t1[c];
+  const int4 ck = pl.chunk[c];
+  const int ft = ck.x, t0 = ck.y, t1 = ck.z, step = ck.w / kStep;
   uint8_t* out = pl.wbuf + (size_t)c * kWChunkBytes;
   // each thread writes 16-byte rows: (freq n, k-group kg) -> 8 transitions
   for (int idx = threadIdx.x; idx < kN * (kKC / 8); idx += blockDim.x) {
@@ -210,7 +228,7 @@ __global__ void __launch_bounds__(256) wgen_kernel(Plan pl, ContractArgs a) {
     float x[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const int t = t0 + kg * 8 + q;
+      const int t = t0 + step * (kg * 8 + q);
       double v = 0.0;
       if (t < t1 && f < a.nf) {
         const bool in = a.window < 0 || abs(f - a.f0[t]) <= a.window;
@@ -236,10 +254,6 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
   const int A = 3 * a.neps;
   const int a0 = tb.x * 8, b0 = tb.y * 8;
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-  // the chunks of an item are consecutive 32-transition slices of one
-  // frequency tile's range
-  const int t_first = nch > 0 ? pl.chunk_t0[c_begin] : 0, t_end = nch > 0 ? pl.chunk_t1[c_begin] : 0;
-
   // overlaps staged per chunk: double-buffered when small (NCH = 1), so that
   // one producer barrier per chunk suffices
   constexpr int kSMBuf = NCH == 1 ? 2 : 1;
@@ -292,12 +306,15 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
       // W chunks whose bulk copy was issued / has landed: on an abort the
       // copies still in flight are waited for before the CTA frees anything
       int issued = -1, landed = -1;
+      int role = nch > 0 ? pl.chunk[c_begin].w : 0;
       for (int n = 0; n < 2 && n < nch; ++n) {
         bulk_load(stage(n) + 2 * kABytes, pl.wbuf + (size_t)(c_begin + n) * kWChunkBytes, kWChunkBytes, &wfull[n]);
         issued = n;
       }
       for (int n = 0; n < nch; ++n) {
-        const int s = n & 1, g = n % pl.flush;
+        const int s = n & 1;
+        const bool zero = (role & kFromZero) != 0;
+        if (n + 1 < nch) role = pl.chunk[c_begin + n + 1].w;
         if (!wait(&afull[s], (n >> 1) & 1, 5) || !wait(&wfull[s], (n >> 1) & 1, 2)) break;
         landed = n;
         tc_fence_after();
@@ -310,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
           const uint64_t alo = umma_desc(sa + kABytes + ks * 2 * (kM / 8) * 128, (kM / 8) * 128, 128);
           const uint64_t bhi = umma_desc(sb + ks * 2 * (kN / 8) * 128, (kN / 8) * 128, 128);
           const uint64_t blo = umma_desc(sb + kBBytes + ks * 2 * (kN / 8) * 128, (kN / 8) * 128, 128);
-          const uint32_t acc0 = (g > 0 || ks > 0) ? 1u : 0u;
+          const uint32_t acc0 = (!zero || ks > 0) ? 1u : 0u;
           mma_bf16(tmem, ahi, bhi, acc0);
           mma_bf16(tmem, ahi, blo, 1u);
           mma_bf16(tmem, alo, bhi, 1u);
@@ -351,22 +368,29 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
     constexpr int kMPer = kKC * 16 * NCH / kProducers;
     float2 mreg[kMPer];
     float wreg = 0.f;
+    int role_next = 0;
+    int4 ck = nch > 0 ? pl.chunk[c_begin] : make_int4(0, 0, 0, 0);  // of the chunk to load next
     auto load_chunk = [&](int n) {
-      const int t0 = t_first + n * kKC;
+      const int t0 = ck.y, t1 = ck.z, step = ck.w / kStep;
 #pragma unroll
       for (int q = 0; q < kMPer; ++q) {
         const int idx = tid + q * kProducers;
         const int t = idx / (16 * NCH), rem = idx % (16 * NCH);
         const int slot = rem / NCH, ch = rem % NCH;
-        const int gt = t0 + t;
+        const int gt = t0 + step * t;
         const int ab = slot < 8 ? a0 + slot : b0 + slot - 8;
-        mreg[q] = (gt < t_end && ab < A) ? M32[((size_t)gt * A + ab) * NCH + ch] : make_float2(0.f, 0.f);
+        mreg[q] = (gt < t1 && ab < A) ? M32[((size_t)gt * A + ab) * NCH + ch] : make_float2(0.f, 0.f);
       }
-      wreg = (tid < kKC && t0 + tid < t_end) ? pl.wgt32[t0 + tid] : 0.f;
+      const int gw = t0 + step * tid;
+      wreg = (tid < kKC && gw < t1) ? pl.wgt32[gw] : 0.f;
+      if (ck.w & kPair2) wreg = -wreg;
+      role_next = ck.w;
+      if (n + 1 < nch) ck = pl.chunk[c_begin + n + 1];
     };
     if (nch > 0) load_chunk(0);
     for (int n = 0; n < nch; ++n) {
-      const int s = n & 1, g = n % pl.flush, sb = kSMBuf == 2 ? s : 0;
+      const int s = n & 1, sb = kSMBuf == 2 ? s : 0;
+      const int role = role_next;
       uint8_t* st = stage(s);
       float2* sMb = sM + sb * kSMElems;
       float* swb = sw + sb * kKC;
@@ -450,14 +474,15 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
       async_proxy_fence();
       if (!(pl.fault == 1 && n == 0)) mbar_arrive(&afull[s]);
       // warps 0-3 (TMEM lanes 0-127) move the FP32 accumulator into the FP64
-      // tile after the group's last chunk: 32 columns at a time through this
+      // tile after a sum's last chunk: 32 columns at a time through this
       // warp's 8 KB of the stage of chunk n (free until chunk n + 2, which
       // waits for these warps), then one bulk copy (first flush) or bulk
       // FP64 add into the tile. A flush starts once the previous one's bulk
       // operations completed, so the additions happen in a fixed order. Their
       // next A-full arrival tells the control warp that the accumulator and
       // the stage may be overwritten.
-      if ((g == pl.flush - 1 || n == nch - 1) && wid < 4) {
+      if ((role & kLast) && wid < 4) {
+        const double weight = (role & kPair2) ? -1.0 : ((role & kPair1) ? 2.0 : 1.0);
         if (wait(&mdone[s], (n >> 1) & 1, 4)) {
           tc_fence_after();
           double* stg = reinterpret_cast<double*>(st) + wid * (32 * 32);
@@ -481,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
             if (lane == 0) bulk_wait_read();
             __syncwarp();
 #pragma unroll
-            for (int q = 0; q < 32; ++q) stg[q * 32 + lane] = (double)__uint_as_float(r[q]);
+            for (int q = 0; q < 32; ++q) stg[q * 32 + lane] = weight * (double)__uint_as_float(r[q]);
             async_proxy_fence();
             __syncwarp();
             if (lane == 0) bulk_store(dst + cb * 32, stg, 32 * 32 * sizeof(double), flushes > 0);
@@ -491,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Plan pl, ContractArg
           tc_fence_before();
         }
       }
-      if (g == pl.flush - 1 || n == nch - 1) ++flushes;
+      if (role & kLast) ++flushes;
     }
     // an empty range (or an abort before the first flush) still owns its
     // tile: the producers zero it
@@ -557,9 +582,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(Plan pl, ContractArgs a) {
 namespace {
 
 struct HostPlan {
-  std::vector<int> chunk_ft, chunk_t0, chunk_t1;
-  int flush = kFlushChunks;
-  std::vector<int4> items;
+  std::vector<int4> chunks, items;
   std::vector<int2> ft_items, tiles;
 };
 
@@ -575,23 +598,36 @@ HostPlan make_plan(const ContractArgs& a, const int2* trange_host, int nft) {
     }
   long long total = 0;
   for (int ft = 0; ft < nft; ++ft) total += (trange_host[ft].y - trange_host[ft].x + kKC - 1) / kKC;
-  if (a.window >= 0 && a.zeros) h.flush = kFlushZeros;
-  // pieces: enough CTAs to fill the GPU a few times, each a multiple of the flush group
+  // pieces: enough CTAs to fill the GPU a few times
   const long long want = std::max<long long>(1, (kTargetCtas + (long long)h.tiles.size() - 1) / h.tiles.size());
-  long long piece = std::max<long long>(kFlushChunks, (total + want - 1) / want);
-  piece = (piece + h.flush - 1) / h.flush * h.flush;
+  long long piece = kKC * std::max<long long>(kMinPiece, (total + want - 1) / want);  // transitions
+  // blocks of an item that are summed separately: all of it in interleaved pairs of
+  // sums, or one sum
+  const bool zeros = a.window >= 0 && a.zeros;
+  const int sum_len = (zeros ? kFlushZeros : kFlushChunks) * kKC;
+  if (!zeros) piece = (piece + sum_len - 1) / sum_len * sum_len;
+  const long long block = zeros ? piece : sum_len;
   h.ft_items.resize(nft);
   for (int ft = 0; ft < nft; ++ft) {
     const int tb = trange_host[ft].x, te = trange_host[ft].y;
-    const int c0 = (int)h.chunk_ft.size();
-    for (int t = tb; t < te; t += kKC) {
-      h.chunk_ft.push_back(ft);
-      h.chunk_t0.push_back(t);
-      h.chunk_t1.push_back(te);
-    }
-    const int c1 = (int)h.chunk_ft.size();
     const int i0 = (int)h.items.size();
-    for (int c = c0; c < c1; c += (int)piece) h.items.push_back(make_int4(ft, c, (int)std::min<long long>(c1, c + piece), 0));
+    for (long long b = tb; b < te; b += piece) {
+      const int c0 = (int)h.chunks.size();
+      const long long e = std::min<long long>(te, b + piece);
+      for (long long t = b; t < e; t += block) {
+        const int end = (int)std::min(e, t + block), len = end - (int)t;
+        const int step = zeros ? 2 * ((len + 2 * sum_len - 1) / (2 * sum_len)) : 1;  // sums of the block
+        const int nh = (len + step * kKC - 1) / (step * kKC);
+        for (int sum = 0; sum < step; ++sum) {
+          const int pair = zeros ? (sum & 1 ? kPair2 : kPair1) : 0;
+          for (int j = 0; j < nh; ++j)
+            h.chunks.push_back(make_int4(ft, (int)t + sum + step * kKC * j, end,
+                                         (j == 0 && pair != kPair2 ? kFromZero : 0) | (j == nh - 1 ? kLast : 0) | pair |
+                                             step * kStep));
+        }
+      }
+      h.items.push_back(make_int4(ft, c0, (int)h.chunks.size(), 0));
+    }
     h.ft_items[ft] = make_int2(i0, (int)h.items.size());
   }
   return h;
@@ -603,12 +639,15 @@ size_t mixed_workspace_bytes(const ContractArgs& a, long long T) {
   // upper bound: every transition in at most ceil((2W+N)/N)+1 frequency tiles
   const int nft = (a.nf + kN - 1) / kN;
   const long long span = a.window < 0 ? nft : std::min<long long>(nft, (2LL * a.window + kN) / kN + 2);
-  const long long nchunk = (T * span + kKC - 1) / kKC + nft + 1;
   const int A = 3 * a.neps, nb = (A + 7) / 8;
   const long long ntile = (long long)nb * nb;
   const long long nitem = kTargetCtas + 2 * nft + 1;  // pieces: want + one remainder per frequency tile
+  // a block of n transitions has at most n / kKC + step chunks, step <= n / (kFlushZeros kKC) + 2,
+  // an item at most one block that is not full
+  const long long full = (T * span + kKC - 1) / kKC;
+  const long long nchunk = full + full / kFlushZeros + 3 * nitem;
   size_t b = 0;
-  b += align256(sizeof(int) * 3 * nchunk);
+  b += align256(sizeof(int4) * nchunk);
   b += align256(sizeof(int4) * nitem);
   b += align256(sizeof(int2) * nft);
   b += align256(sizeof(int2) * ntile);
@@ -689,7 +728,7 @@ cudaError_t launch_contract_mixed(const ContractArgs& a, long long T, void* ws, 
   Plan pl{};
   pl.nft = nft;
   pl.ntile = (int)h.tiles.size();
-  pl.nchunk = (int)h.chunk_ft.size();
+  pl.nchunk = (int)h.chunks.size();
   pl.nitem = (int)h.items.size();
   const int A = 3 * a.neps;
   uint8_t* p = reinterpret_cast<uint8_t*>(ws);
@@ -698,10 +737,7 @@ cudaError_t launch_contract_mixed(const ContractArgs& a, long long T, void* ws, 
     p += align256(bytes);
     return r;
   };
-  pl.chunk_ft = reinterpret_cast<int*>(take(sizeof(int) * std::max(1, pl.nchunk)));
-  pl.chunk_t0 = reinterpret_cast<int*>(take(sizeof(int) * std::max(1, pl.nchunk)));
-  pl.chunk_t1 = reinterpret_cast<int*>(take(sizeof(int) * std::max(1, pl.nchunk)));
-  pl.flush = h.flush;
+  pl.chunk = reinterpret_cast<int4*>(take(sizeof(int4) * std::max(1, pl.nchunk)));
   pl.item = reinterpret_cast<int4*>(take(sizeof(int4) * std::max(1, pl.nitem)));
   pl.ft_items = reinterpret_cast<int2*>(take(sizeof(int2) * nft));
   pl.tiles = reinterpret_cast<int2*>(take(sizeof(int2) * std::max(1, pl.ntile)));
@@ -720,9 +756,7 @@ cudaError_t launch_contract_mixed(const ContractArgs& a, long long T, void* ws, 
     e = cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st);                                     \
     if (e != cudaSuccess) return e;                                                                   \
   }
-  PMX_CP(pl.chunk_ft, h.chunk_ft.data(), sizeof(int) * pl.nchunk);
-  PMX_CP(pl.chunk_t0, h.chunk_t0.data(), sizeof(int) * pl.nchunk);
-  PMX_CP(pl.chunk_t1, h.chunk_t1.data(), sizeof(int) * pl.nchunk);
+  PMX_CP(pl.chunk, h.chunks.data(), sizeof(int4) * pl.nchunk);
   PMX_CP(pl.item, h.items.data(), sizeof(int4) * pl.nitem);
   PMX_CP(pl.ft_items, h.ft_items.data(), sizeof(int2) * nft);
   PMX_CP(pl.tiles, h.tiles.data(), sizeof(int2) * pl.ntile);
