@@ -201,14 +201,15 @@ namespace {
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
-  ~DevBuf() {
-    if (ptr) cudaFree(ptr);
-  }
-  cudaError_t ensure(size_t b) {
-    if (b <= bytes) return cudaSuccess;
+  ~DevBuf() { release(); }
+  void release() {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     bytes = 0;
+  }
+  cudaError_t ensure(size_t b) {
+    if (b <= bytes) return cudaSuccess;
+    release();
     cudaError_t e = cudaMalloc(&ptr, b);
     if (e == cudaSuccess) bytes = b;
     return e;
@@ -221,14 +222,16 @@ struct DevBuf {
 
 struct CudaFail : std::runtime_error {
   int code;
-  CudaFail(const std::string& m, int c) : std::runtime_error(m), code(c) {}
+  bool no_memory;
+  CudaFail(const std::string& m, int c, bool oom = false) : std::runtime_error(m), code(c), no_memory(oom) {}
 };
 
 #define CK(x)                                                                                        \
   do {                                                                                               \
     cudaError_t e_ = (x);                                                                            \
     if (e_ != cudaSuccess)                                                                           \
-      throw CudaFail(std::string(#x) + ": " + cudaGetErrorString(e_), PMX_ERR_CUDA);                 \
+      throw CudaFail(std::string(#x) + ": " + cudaGetErrorString(e_), PMX_ERR_CUDA,                  \
+                     e_ == cudaErrorMemoryAllocation);                                               \
   } while (0)
 
 }  // namespace
@@ -276,6 +279,7 @@ struct pmx_ctx {
   DevBuf a_lam, a_C, a_X, a_R, a_SV, a_SSO, a_kp, a_linv, a_tri, a_work;
   // several crystals at once (batched entry points)
   DevBuf b_g, b_hkl, b_vloc, b_vso, b_crystal;
+  bool lean = false;                   // second run of a call that ran out of device memory (see guarded)
   int kk_nf = 0;                       // grid length of the Kramers-Kronig tables in kktab (0: none)
   double m2_err = 0.0, m2_max = 0.0;  // |M|^2 error of the mixed path's FP32 overlaps (last call)
   long long mixed_mmas = 0;            // tcgen05 MMA instructions of the mixed contractions so far
@@ -339,21 +343,37 @@ void collect_ktimes(pmx_ctx* c) {
   c->kpending.clear();
 }
 
+// Runs one entry point. The large workspaces (H, reflectors and scratch of as many
+// eigenproblems as fill the GPU, the vectors of a group of q, the table of line shapes)
+// are sized for speed and stay in the context; a call for which the device has no room
+// left, or that finds it taken by them, gives them back and is run once more from the
+// start with the smallest ones (ctx->lean). Every f must therefore be able to run twice:
+// results and sums of an entry point are written or reset on the way.
 template <class F>
 int guarded(pmx_ctx* ctx, F&& f) {
   if (!ctx) return PMX_ERR_INVALID;
-  ctx->err.clear();
-  try {
-    CK(cudaSetDevice(ctx->device));
-    const int rc = f();
-    collect_ktimes(ctx);
-    return rc;
-  } catch (const CudaFail& e) {
-    ctx->err = e.what();
-    return e.code;
-  } catch (const std::exception& e) {
-    ctx->err = e.what();
-    return PMX_ERR_INVALID;
+  for (ctx->lean = false;; ctx->lean = true) {
+    ctx->err.clear();
+    try {
+      CK(cudaSetDevice(ctx->device));
+      const int rc = f();
+      collect_ktimes(ctx);
+      return rc;
+    } catch (const CudaFail& e) {
+      if (e.no_memory) {
+        cudaGetLastError();  // a later launch must not find this error
+        cudaStreamSynchronize(ctx->stream);
+        for (DevBuf* b : {&ctx->hbuf, &ctx->rbuf, &ctx->scratch, &ctx->zk, &ctx->zq, &ctx->c64ws, &ctx->mixws,
+                          &ctx->a_zb, &ctx->a_C, &ctx->a_X, &ctx->a_work})
+          b->release();
+        if (!ctx->lean) continue;
+      }
+      ctx->err = e.what();
+      return e.code;
+    } catch (const std::exception& e) {
+      ctx->err = e.what();
+      return PMX_ERR_INVALID;
+    }
   }
 }
 
@@ -476,10 +496,11 @@ cudaError_t eig_launch(pmx_ctx* c, const pmx::dev::EigItem* items, int nitems, i
 // waves of 148 matrices of the largest size need more (n > 832), so that the
 // large sizes still fill the GPU; 4 GB and one matrix more where the reduction is
 // kept, whose caller keeps 2 GB at k and k + q each and the reference point
-// within one chunk
-size_t h_budget(size_t hbytes_max, bool keep) {
-  const size_t base = (size_t)2 << 30;
-  return keep ? 2 * base + hbytes_max : std::max(base, std::min((size_t)8 << 30, 296 * hbytes_max));
+// within one chunk. 64 MB, or one matrix, where memory has run out
+size_t h_budget(const pmx_ctx* c, size_t hbytes_max, bool keep) {
+  const size_t base = (size_t)(c->lean ? 64 : 2048) << 20;
+  if (keep) return 2 * std::max(base, hbytes_max) + hbytes_max;
+  return c->lean ? base : std::max(base, std::min((size_t)8 << 30, 296 * hbytes_max));
 }
 
 // One set of eigenproblems of a crystal: H(k) of every k, the lowest nval
@@ -517,7 +538,7 @@ void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& s
   const bool tri_req = tri != nullptr;
   const int ld = eig_ld(n, n, tri_req);
   const size_t hbytes = (size_t)ld * ld * sizeof(double2);
-  int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nk, h_budget(hbytes, keep) / hbytes));
+  int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nk, h_budget(c, hbytes, keep) / hbytes));
   chunk = std::min(chunk, 4096);
   if (keep && nk > chunk) throw CudaFail("the adjoint's block does not fit one eigensolver chunk", PMX_ERR_LIMIT);
   if (nk > chunk) {  // several chunks: each a whole number of waves of CTAs
@@ -1391,7 +1412,7 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
       ctx->launches += 1;
     } else if (precision == PMX_PREC_FP64) {
       // without the memory for the table of line shapes the kernel forms them itself
-      bool table = pmx::dev::contract64_wants_table(ca, Tn);
+      bool table = !ctx->lean && pmx::dev::contract64_wants_table(ca, Tn);
       if (table && ctx->c64ws.ensure(pmx::dev::contract64_workspace_bytes(ca, Tn, true)) != cudaSuccess) {
         cudaGetLastError();
         table = false;
@@ -1498,7 +1519,8 @@ static int run_chi(pmx_ctx* ctx, const pmx_problem* P, int sw, int precision, do
     // eigenvectors at k, then at k + q of a group of q's: as many q's as make about
     // eight waves of 148 matrices with the k points, within 4 GB
     const long long zq = (long long)nk * nev * n;
-    const long long zfit = ((long long)4 << 30) / std::max<long long>(1, zq * (long long)sizeof(double2));
+    const long long zfit =
+        ctx->lean ? 1 : ((long long)4 << 30) / std::max<long long>(1, zq * (long long)sizeof(double2));
     const int group = (int)std::max<long long>(
         1, std::min<long long>({(long long)pl.nq, (8 * 148 + nk - 1) / std::max(1, nk), zfit}));
     CK(ctx->zk.ensure(std::max<size_t>(sizeof(double2) * (size_t)(1 + group) * zq, 16)));
@@ -2003,7 +2025,7 @@ extern "C" int pmx_band_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* dE
     double osum = 0.0;
     if (nkeep > 0 && nq > 0) {
       const int ns = solved_states(nkeep, dc.soc), n = dc.n;
-      const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nq, ((size_t)1 << 30) / ((size_t)ns * n * 16)));
+      const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nq, ((size_t)(ctx->lean ? 64 : 1024) << 20) / ((size_t)ns * n * 16)));
       // the reference point is solved with the first chunk, unless its gradient is zero
       for (int q = 0; q < nq; ++q)
         for (int s = 0; s < nkeep; ++s) osum += dE[(size_t)q * p.nband + s];
@@ -2099,7 +2121,8 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
     const bool two_stage = use_two_stage(n, false);
     const int ld = eig_ld(n, n, !two_stage);
     const int kb = (int)std::max<size_t>(
-        1, std::min<size_t>({(size_t)nk, ((size_t)2 << 30) / ((size_t)ld * ld * 16), (size_t)2047}));
+        1, std::min<size_t>({(size_t)nk, ((size_t)(ctx->lean ? 64 : 2048) << 20) / ((size_t)ld * ld * 16),
+                                               (size_t)2047}));
     (void)nall;
     CK(ctx->a_kk.ensure(sizeof(double) * 2 * (size_t)np * nf));
     CK(ctx->chi2.ensure(sizeof(double) * 2 * (size_t)np * nf));
@@ -2493,7 +2516,7 @@ void solve_multi(pmx_ctx* c, const pmx::dev::CrystalDev* table, std::vector<Solv
   while (i0 < order.size()) {
     const int max_n = reqs[order[i0]].n, cls = heev_class(max_n);
     const size_t ld0 = (size_t)eig_ld(max_n, max_n, false);
-    const size_t hmax = h_budget(ld0 * ld0 * sizeof(double2), false);
+    const size_t hmax = h_budget(c, ld0 * ld0 * sizeof(double2), false);
     size_t i1 = i0, hb = 0;
     while (i1 < order.size() && i1 - i0 < 4096 && heev_class(reqs[order[i1]].n) == cls) {
       const size_t ldi = (size_t)eig_ld(reqs[order[i1]].n, max_n, false);
@@ -2715,7 +2738,7 @@ extern "C" int pmx_chi_batch(pmx_ctx* ctx, int count, const pmx_problem* const* 
     std::vector<ChiPlan> pl;
     for (int i = 0; i < count; ++i) pl.push_back(chi_plan(problems[i]->p, sw, set.dc[i]));
     // groups of problems whose eigenvectors at k and at k+q (one q) fit the budget
-    const size_t budget = (size_t)16 << 30;
+    const size_t budget = (size_t)(ctx->lean ? 1 : 16) << 30;
     int g0 = 0;
     while (g0 < count) {
       int g1 = g0;
