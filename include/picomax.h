@@ -176,8 +176,9 @@ int pmx_ctx_set_autotune(pmx_ctx* ctx, int on);
 /* Fixes the eigensolver schedule (0 = the two-stage solver where it applies,
  * n >= 96, then the one-stage schedules the matrix size allows: direct loads,
  * prefetch rings, shared-memory partials; an index beyond the last one means
- * the last) for every later batch; -1 returns to the
- * autotuner. For tests that compare the schedules. No reference counterpart. */
+ * the last) for every later batch, the adjoint's reductions among them; -1
+ * returns to the autotuner (and the adjoint to 0 where that is the two-stage
+ * solver). For tests that compare the schedules. No reference counterpart. */
 int pmx_ctx_set_schedule(pmx_ctx* ctx, int schedule);
 /* The autotuner's choices and trial times as JSON text (NUL-terminated,
  * truncated at len; full length in *needed). */

@@ -519,8 +519,9 @@ struct SolveSet {
 // fill. zdev may be null when no set has vectors.
 // With keep the reduction H = Q T Q^H of every item stays behind for the adjoint (all
 // sets must then fit one chunk, see h_budget): of the two-stage solver in c->hbuf and
-// c->rbuf, items in set order; below its sizes of the one-stage one, reflectors in
-// c->hbuf and the tridiagonal form in tri (device, [items][4 n]).
+// c->rbuf, items in set order; outside its sizes, or where a one-stage schedule is
+// fixed, of the one-stage one, reflectors in c->hbuf and the tridiagonal form in tri
+// (device, [items][4 n]).
 void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& sets, double2* zdev,
                 bool keep = false, double* tri = nullptr) {
   const int n = dc.n;
@@ -594,10 +595,12 @@ void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& s
     int variant = 0;
     const int nvar = eig_variants(n, nval, tri_req);
     auto it_choice = c->heev_choice.find(key);
-    if (keep) {
-      variant = 0;  // the two-stage solver where it applies
+    if (keep && !tri_req) {
+      variant = 0;  // the caller asked for the two-stage reduction
     } else if (c->fixed_schedule >= 0) {
-      variant = std::min(c->fixed_schedule, nvar - 1);
+      // with tri only the one-stage schedules are counted
+      const int skip = tri_req && use_two_stage(n, false) ? 1 : 0;
+      variant = std::min(std::max(c->fixed_schedule - skip, 0), nvar - 1);
     } else if (it_choice != c->heev_choice.end()) {
       variant = it_choice->second;
     } else if (nvar > 1 && c->autotune && cnt >= 148) {
@@ -2118,7 +2121,7 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
     // of the rest; a block's reflectors must fit one eigensolver chunk.
     int nsx = std::min(n, ns + 8);
     // (2 kb + 1 matrices make one eigensolver chunk, at most 4096)
-    const bool two_stage = use_two_stage(n, false);
+    const bool two_stage = use_two_stage(n, false) && ctx->fixed_schedule <= 0;
     const int ld = eig_ld(n, n, !two_stage);
     const int kb = (int)std::max<size_t>(
         1, std::min<size_t>({(size_t)nk, ((size_t)(ctx->lean ? 64 : 2048) << 20) / ((size_t)ld * ld * 16),
