@@ -29,8 +29,12 @@ constexpr int kTriInvIters = 3;
 // itself, not of its ratios p_i / p_{i-1}: the ratios take a division per row, on
 // the chain from row to row (90 cycles), the sequence one FMA (8). It is the exact
 // sequence of a T whose entries differ by rounding errors of d - x and e^2, as the
-// ratios are. Every 8 rows both running terms are scaled by a power of two (a row
-// grows them by at most 3 and shrinks them by at least 1e-30). A zero counts as
+// ratios are. Every 8 rows both running terms are scaled by a power of two, and the
+// smaller one raised to 2^-200 of the larger (a change of d by less). In between they
+// stay in range: a row grows them by 3 at most, and since d - x is zero or above 2^-100
+// and e^2 zero or above 2^-172 (tri_snap, tri_eigvals) a row shrinks them by 1e-30 at
+// most, two rows by 1e-52. Without this, a chain of d = x and tiny e ran into
+// zeros. A zero counts as
 // positive: its neighbours have opposite signs, so exactly one change is seen; only
 // after a zero off-diagonal would it wipe out the rest, so with SPLIT (some e2 is
 // zero) zeros are replaced by tiny values of the sign opposite to the last one.
@@ -54,12 +58,16 @@ __device__ __forceinline__ int sturm_count(const double* d, const double* e2, in
     // 2^-exponent of the larger one
     const int ex = max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff);
     const double sc = __hiloint2double((2046 - min(max(ex, 1), 2045)) << 20, 0);
-    p0 *= sc;
-    p1 *= sc;
+    p0 = copysign(fmax(fabs(p0 * sc), 0x1p-200), p0);
+    p1 = copysign(fmax(fabs(p1 * sc), 0x1p-200), p1);
   }
   for (; i < n; ++i) row(i);
   return c;
 }
+
+// A value of the scaled T or a probe, rounded to a multiple of 2^-97 (if it is above
+// 2^-48 it is one of 2^-100 already): far below the bisection's 2^-76.
+__device__ __forceinline__ double tri_snap(double v) { return fabs(v) < 0x1p-48 ? (v + 0x1.8p-45) - 0x1.8p-45 : v; }
 
 __device__ __forceinline__ double hash_uniform(unsigned long long a, unsigned long long b) {
   unsigned long long x = a * 0x9E3779B97F4A7C15ull ^ (b + 0x632BE59BD9B4E019ull);
@@ -145,11 +153,11 @@ __device__ inline int tri_eigvals(const TriWork& W, int n, int nval, double* __r
     double v = e[i];
     if (fabs(v) <= DBL_EPSILON * (fabs(d[i]) + fabs(d[i + 1]))) e[i] = v = 0.0;
     v = scalbn(v, -ex);
-    e2[i] = v * v;
+    e2[i] = fabs(v) < 0x1p-86 ? 0.0 : v * v;
     split |= e2[i] == 0.0;
   }
   split = __syncthreads_or(split);
-  for (int i = tid; i < n; i += nthr) d[i] = scalbn(d[i], -ex);
+  for (int i = tid; i < n; i += nthr) d[i] = tri_snap(scalbn(d[i], -ex));
   const double pad = 2.0 * DBL_EPSILON * n + DBL_MIN;
   const double glo = scalbn(red[0], -ex) - pad, ghi = scalbn(red[1], -ex) + pad;
   // brackets end at 2 eps |lambda|, at least 2^-24 eps of the norm
@@ -172,7 +180,7 @@ __device__ inline int tri_eigvals(const TriWork& W, int n, int nval, double* __r
         double l = lo[k], h = hi[k];
         const double tol = tol_of(l, h);
         if (h - l > tol) {
-          const double x = l + 0.5 * (h - l);
+          const double x = tri_snap(l + 0.5 * (h - l));
           if (sturm_count(W, n, x, split) <= k)
             l = x;
           else
@@ -193,12 +201,12 @@ __device__ inline int tri_eigvals(const TriWork& W, int n, int nval, double* __r
     // the first round's probes cover the whole interval for every eigenvalue
     const int k = tid / G, g = tid % G;
     if (iter == 0) {
-      const double x = glo + (ghi - glo) * (double)(tid + 1) / (double)(nthr + 1);
+      const double x = tri_snap(glo + (ghi - glo) * (double)(tid + 1) / (double)(nthr + 1));
       xs[tid] = x;
       cnt[tid] = sturm_count(W, n, x, split);
     } else if (k < nval) {
       const double l = lo[k], h = hi[k];
-      const double x = l + (h - l) * (double)(g + 1) / (double)(G + 1);
+      const double x = tri_snap(l + (h - l) * (double)(g + 1) / (double)(G + 1));
       xs[tid] = x;
       cnt[tid] = sturm_count(W, n, x, split);
     }
