@@ -646,7 +646,8 @@ __global__ void __launch_bounds__(kThr, OCC) sb_kernel(const EigItem* __restrict
 //   E  E(s, j) H applied, reflector j + 1 formed: 2 j + 1; E(s, j) done: 2 (j + 1)
 // D(s, j) needs E(s-1, j) and D(s-1, j+1); E(s, j) needs those and only the first
 // half of E(s-1, j+1), of whose block it touches one element, the corner (first
-// row and column) that is final then. Within a sweep D(s, j) waits for E's
+// row and column) that is final then (tests/test_bulge_order.py holds every access of
+// every task against these waits). Within a sweep D(s, j) waits for E's
 // reflector, and E, before it writes a reflector slot, for D to have left it. No
 // barrier of any kind between steps.
 //
@@ -775,9 +776,10 @@ __global__ void __launch_bounds__(64 * kPairs, kMaxPairs / kPairs) sbtrd_kernel(
     doff[cc] = c <= i ? c * (kBandLd - 1) + i : i * (kBandLd - 1) + c;
     if (c > i) up |= 1u << cc;
   }
-  // E element (i, 8h + cc) at e_off + cc (kBandLd - 1); (8h + rr, column i) at t_off + rr
+  // E element (i, 8h + cc) at e_off + cc (kBandLd - 1); (8h + rr, column i) at t_off + rr, for
+  // i = 0 column 1 again: column 0 is final there, and the next sweep may be writing its corner
   const int e_off = 8 * h * (kBandLd - 1) + kNB + i;
-  const int t_off = i * (kBandLd - 1) + kNB + 8 * h;
+  const int t_off = max(i, 1) * (kBandLd - 1) + kNB + 8 * h;
   for (int s = pair; s <= ld - 2; s += kPairs) {
     const int ns = sweep_steps(ld, s), nprev = s > 0 ? sweep_steps(ld, s - 1) : 0;
     const int base = s * kProgStride, pbase = (s - 1) * kProgStride, pp = (s - 1) & (kPairs - 1);
