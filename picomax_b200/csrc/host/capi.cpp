@@ -511,6 +511,7 @@ struct SolveSet {
   int nval, nvec;
   long long z_off;
   std::vector<double>* w;
+  std::string what = "k-point";  // of an item, in errors
 };
 
 // Assembles and diagonalises H(k) of all sets in common launches: the solver's
@@ -635,8 +636,8 @@ void solve_sets(pmx_ctx* c, const DevCrystal& dc, const std::vector<SolveSet>& s
     c->d2h += sizeof(int) * cnt;
     for (int i = 0; i < cnt; ++i)
       if (info[i] != 0)
-        throw CudaFail("eigensolver failed (status " + std::to_string(info[i]) + ") at k-point " +
-                           std::to_string(where[k0 + i].second),
+        throw CudaFail("eigensolver failed (status " + std::to_string(info[i]) + ") at " +
+                           sets[where[k0 + i].first].what + " " + std::to_string(where[k0 + i].second),
                        eig_status_error(info[i]));
   }
   std::vector<double> w((size_t)nk * nval);
@@ -657,21 +658,24 @@ inline double spinor_eig(const std::vector<double>& w, int nev, int k, int s, in
 // Number of solved states needed to cover `spinor` spinor states.
 inline int solved_states(int spinor, int soc) { return soc ? spinor : (spinor + 1) / 2; }
 
+std::string kq_name(int q) { return "k + q (q " + std::to_string(q) + "), k-point"; }
+
 // The eigenproblem of the reference energy (setRefEnergy, src/pmx_epm.cpp:393-428)
 // as a set of a solve, empty when nvalence is out of bounds, and the energy from
 // its eigenvalues.
 struct RefSolve {
   int nev = 0;
   std::vector<double> w;
+  static constexpr const char* what = "reference point";
   SolveSet set(const Problem& p, int soc, int nvec = 0, long long z_off = 0) {
     const int nh = 2 * p.npw();
     if (!(p.nvalence > 0 && p.nvalence < nh)) {
       std::cout << "WARNING::setRefEnergy:: nvalence is out of bounds for eigenvalues. Setting offset to 0."
                 << std::endl;
-      return {{}, 0, 0, 0, &w};
+      return {{}, 0, 0, 0, &w, what};
     }
     nev = solved_states(p.nvalence + 1, soc);
-    return {{p.refpoint}, nev, nvec, z_off, &w};
+    return {{p.refpoint}, nev, nvec, z_off, &w, what};
   }
   double energy(const Problem& p, int soc) const {
     if (nev == 0) return 0.0;
@@ -839,7 +843,7 @@ extern "C" int pmx_band(pmx_ctx* ctx, const pmx_problem* P, double* eband) {
     }
     const int nev = solved_states(nkeep, dc.soc);
     std::vector<double> w;
-    solve_sets(ctx, dc, {ref_set, {p.lat.Q, nev, 0, 0, &w}}, nullptr);
+    solve_sets(ctx, dc, {ref_set, {p.lat.Q, nev, 0, 0, &w, "q-point"}}, nullptr);
     const double off = ref.energy(p, dc.soc);
     for (int q = 0; q < p.nq(); ++q)
       for (int n = 0; n < p.nband; ++n)
@@ -1544,7 +1548,7 @@ static int run_chi(pmx_ctx* ctx, const pmx_problem* P, int sw, int precision, do
         for (int i = 0; i < cnt; ++i) {
           std::vector<Vec3> kq(nk);
           for (int k = 0; k < nk; ++k) kq[k] = p.K[k] + p.lat.Q[q0 + i];
-          sets.push_back({std::move(kq), nval, nev, (1 + i) * zq, &wq[i]});
+          sets.push_back({std::move(kq), nval, nev, (1 + i) * zq, &wq[i], kq_name(q0 + i)});
         }
         solve_sets(ctx, dc, sets, ctx->zk.as<double2>());
         if (q0 == 0) off = ref.energy(p, dc.soc);
@@ -2040,8 +2044,8 @@ extern "C" int pmx_band_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* dE
         const int cnt = std::min(chunk, nq - q0);
         std::vector<Vec3> ks(p.lat.Q.begin() + q0, p.lat.Q.begin() + q0 + cnt);
         std::vector<double> w, wref;
-        std::vector<SolveSet> sets{{ks, ns, ns, 0, &w}};
-        if (q0 == 0 && with_ref) sets.push_back({{p.refpoint}, rs, rs, zref, &wref});
+        std::vector<SolveSet> sets{{ks, ns, ns, 0, &w, "q-point " + std::to_string(q0) + " +"}};
+        if (q0 == 0 && with_ref) sets.push_back({{p.refpoint}, rs, rs, zref, &wref, RefSolve::what});
         solve_sets(ctx, dc, sets, ctx->zq.as<double2>());
         std::vector<double> lb((size_t)cnt * ns, 0.0);
         for (int q = 0; q < cnt; ++q)
@@ -2174,7 +2178,8 @@ extern "C" int pmx_epsm_vjp(pmx_ctx* ctx, const pmx_problem* P, const double* ch
           if (!two_stage) CK(ctx->a_tri.ensure(sizeof(double) * 4 * (size_t)(2 * cnt + 1) * n));
           {
             Timer tm(ctx, 0);
-            std::vector<SolveSet> sets{{ks, nvl, nvs, 0, &wk}, {kqs, nvl, nvs, zs, &wq}};
+            std::vector<SolveSet> sets{{ks, nvl, nvs, 0, &wk, "k-point " + std::to_string(k0) + " +"},
+                                       {kqs, nvl, nvs, zs, &wq, kq_name(q) + " " + std::to_string(k0) + " +"}};
             const bool first = ref.w.empty() && !ref_set.ks.empty();
             if (first) sets.push_back(ref_set);
             solve_sets(ctx, dc, sets, ctx->zk.as<double2>(), true, two_stage ? nullptr : ctx->a_tri.as<double>());
