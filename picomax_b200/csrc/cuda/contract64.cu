@@ -325,6 +325,7 @@ int grid_blocks(const ContractArgs& a) {
 // frequencies) leave SMs idle, so that their transitions are cut until about two
 // waves of two CTAs per SM run, each with 8 chunks or more.
 int contract64_split(const ContractArgs& a, long long T) {
+  if (a.one_share) return 1;
   const long long ctas = (long long)grid_blocks(a) * ((a.nf + kFT - 1) / kFT);
   const long long want = (4 * 148 + ctas - 1) / std::max(1LL, ctas);
   return (int)std::max(1LL, std::min({want, (long long)kMaxSplit, T / (8 * kTK)}));

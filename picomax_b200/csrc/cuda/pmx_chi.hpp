@@ -101,6 +101,7 @@ struct ContractArgs {
   int neps, np, nf, nch;
   int window;           // half width, or -1 for all frequencies
   int zeros;            // the window only leaves out zeros of the line shape
+  int one_share;        // FP64: no partial sums (no memory for them)
   int delta;            // broadening model
   double eps, dfreq;
   double* acc;          // [2][9][np][nf] Re then Im

@@ -1405,6 +1405,7 @@ void chi_process_q(pmx_ctx* ctx, const Problem& p, const ChiPlan& pl, const DevC
     ca.nch = nch;
     ca.window = W;
     ca.zeros = mode != 0 ? 1 : 0;
+    ca.one_share = ctx->lean ? 1 : 0;
     ca.delta = p.delta;
     ca.eps = p.epsilon;
     ca.dfreq = p.dfreq;
