@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(kCThreads) contract_pv_kernel(ContractArgs a) 
   WTile* sW = reinterpret_cast<WTile*>(sP2 + kPairs);
   double* sw = reinterpret_cast<double*>(sW + 4);
   double* sde = sw + kTK;
-  int* sf0 = reinterpret_cast<int*>(sde + kTK);
   const int tid = threadIdx.x;
   const int pg = tid / 16, fg = tid % 16;
   double acc1[9][4], acc2[9][4];  // 1: Im (reO), 2: Re (-imO)
@@ -276,7 +275,6 @@ __global__ void __launch_bounds__(kCThreads) contract_pv_kernel(ContractArgs a) 
       const int t = tid;
       sw[t] = t < nt ? a.wgt[t0 + t] : 0.0;
       sde[t] = t < nt ? a.dE[t0 + t] : 0.0;
-      sf0[t] = t < nt ? a.f0[t0 + t] : 0;
     }
     __syncthreads();
     // pair products P1 = w reO, P2 = -w imO
@@ -292,13 +290,12 @@ __global__ void __launch_bounds__(kCThreads) contract_pv_kernel(ContractArgs a) 
       const int t = idx / kFT, fl = idx % kFT;
       const int f = f_lo + fl;
       double wv = 0.0;
-      const bool in = t < nt && f < a.nf && (a.window < 0 || abs(f - sf0[t]) <= a.window);
       const double om = a.dfreq * f;
-      if (in) wv = broaden(a.delta, a.eps, sde[t] - om);
+      const bool ok = t < nt && f < a.nf;
+      if (ok) wv = broaden(a.delta, a.eps, sde[t] - om);
       sW[0][t][fl] = wv;
       const double de = sde[t];
       const double den = de * de - om * om;
-      const bool ok = t < nt && f < a.nf;
       sW[1][t][fl] = ok ? de / den : 0.0;          // LL
       sW[2][t][fl] = ok ? 1.0 / den : 0.0;         // LT
       sW[3][t][fl] = ok ? 1.0 / de / den : 0.0;    // TT
@@ -355,8 +352,7 @@ cudaError_t launch_contract_pv(const ContractArgs& a, cudaStream_t st) {
   dim3 grid(ntiles, nft);
   if (a.nch != 1 || !a.acc_pv) return cudaErrorInvalidValue;
   const size_t sm = (size_t)2 * kTK * kAB * sizeof(double2) + (size_t)2 * kPairs * (kTK + 1) * sizeof(double) +
-                    (size_t)4 * kTK * kFT * sizeof(double) + (size_t)2 * kTK * sizeof(double) +
-                    (size_t)kTK * sizeof(int);
+                    (size_t)4 * kTK * kFT * sizeof(double) + (size_t)2 * kTK * sizeof(double);
   const cudaError_t err =
       cudaFuncSetAttribute(contract_pv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (err != cudaSuccess) return err;

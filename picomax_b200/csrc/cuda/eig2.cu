@@ -1,9 +1,9 @@
 // Two-stage batched FP64 Hermitian eigensolver: dense -> band -> tridiagonal.
 //
 // Replaces Eigen::SelfAdjointEigenSolver (src/pmx_epm.cpp:232, :402,
-// src/pmx_chi.cpp:388, :476) for the sizes whose matrix does not fit in
-// shared memory. The one-stage reduction (epm.cu) streams the whole trailing
-// block through L2/HBM once per column; here the Householder reduction is
+// src/pmx_chi.cpp:388, :476) for n from 96 up to a padded size of 1216. The
+// one-stage reduction (epm.cu) passes over the whole trailing block once per
+// column; here the Householder reduction is
 // split the way blocked LAPACK/PLASMA solvers split it (Bischof, Lang, Sun,
 // "A framework for symmetric band reduction", ACM TOMS 26 (2000); Haidar,
 // Ltaief, Dongarra, SC'11), each stage B200-shaped:
@@ -24,7 +24,8 @@
 //  2. sbtrd_kernel (one CTA per matrix): the band (16 sub-diagonals plus 16
 //     for the bulge) lives in shared memory up to ld = 416, beyond that in
 //     the item's slot of the reflector buffer (L1/L2); sweeps chase their bulges down
-//     the band, eight at a time (a pair of warps per sweep), each step of a
+//     the band, eight at a time (four in large batches of small matrices; a pair of
+//     warps per sweep), each step of a
 //     sweep waiting only for the previous sweep to leave its rows (progress
 //     words in shared memory, no block-wide barrier). Reflectors go to
 //     global memory.

@@ -22,7 +22,6 @@
 
 #include "pmx_common.cuh"
 #include "pmx_device.hpp"
-#include "pmx_tri.cuh"
 #include "pmx_trieig.cuh"
 
 namespace pmx {

@@ -1,5 +1,4 @@
-// Tridiagonal solve shared by the eigensolver (inverse iteration) and the
-// adjoint (resolvent of T).
+// Tridiagonal solve of the adjoint's resolvent on the one-stage reduction.
 #pragma once
 
 #include <cuda_runtime.h>
