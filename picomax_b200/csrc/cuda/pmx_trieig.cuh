@@ -250,6 +250,9 @@ __device__ inline int tri_eigvals(const TriWork& W, int n, int nval, double* __r
 // the multiplier f (its lowest mantissa bit set when rows i and i + 1 were
 // swapped, a change of one unit in the last place of f) and 1 / pivot, at
 // [i * st]. U's two super-diagonals follow from f, d and e (tri_factored_solve).
+// Pivots are kept at or above `tiny` (eps |T|): the eigenvalues of a cluster may be
+// equal, and a solve that amplified one of its directions by far more than the others
+// would leave the cluster's iterates parallel (graded T: no orthogonality, or NaN).
 __device__ inline void tri_factor(const double* __restrict__ d, const double* __restrict__ e, int n, double lam,
                                   double tiny, double* __restrict__ F, double* __restrict__ I0, int st) {
   double a = d[0] - lam;          // current pivot-row diagonal
@@ -257,8 +260,8 @@ __device__ inline void tri_factor(const double* __restrict__ d, const double* __
   for (int i = 0; i < n - 1; ++i) {
     const double b = e[i], dn = d[i + 1] - lam, en = i + 1 < n - 1 ? e[i + 1] : 0.0;
     const size_t o = (size_t)i * st;
-    if (fabs(a) >= fabs(b)) {
-      if (a == 0.0) a = tiny;
+    if (fabs(a) >= fabs(b) || fabs(b) < tiny) {
+      if (fabs(a) < tiny) a = copysign(tiny, a);
       const double ia = 1.0 / a, f = b * ia;
       F[o] = __longlong_as_double(__double_as_longlong(f) & ~1ll);
       I0[o] = ia;
@@ -272,7 +275,7 @@ __device__ inline void tri_factor(const double* __restrict__ d, const double* __
       c = -f * en;
     }
   }
-  if (a == 0.0 || fabs(a) < tiny) a = a < 0 ? -tiny : tiny;
+  if (fabs(a) < tiny) a = copysign(tiny, a);
   I0[(size_t)(n - 1) * st] = 1.0 / a;
 }
 
