@@ -192,20 +192,21 @@ __host__ __device__ inline size_t sb_smem_bytes(int ld, int mr, bool yg, bool vg
 // |x|^2, for c < j (conjugated) the dot v_c^H v_j of the T column (zlarft).
 // The two row groups of a warp are summed with one shuffle, the eight warps'
 // sums in shared memory. The update of the columns has one form for every
-// column, a_c[r] -= a_j[r] s_c (s_c = scal w_c for c > j, 1 - scal for c = j,
-// 0 for c < j), so that the lanes of a warp do not diverge. Rows go four at a
+// column, a_c[r] -= a_j[r] s_c (s_c = scal w_c for c > j, else 0), so that the lanes
+// of a warp do not diverge; the columns keep a_c unscaled and become v_c = scal a_c at
+// the end (a_c - a_c (1 - scal) lost eps |A| of v_c, all of it at |A| = 1e16). Rows go four at a
 // time (slots past the panel hold zeros), so that four loads of the pivot column
 // and four chains are in flight: with a check per row the two warps of a scheduler
 // waited for one load after another at large n. The pivot column reaches the threads of a row group through the warp's own shared-memory buffer (the
 // group's 16 threads share a warp). red/rowj: [2][8][16] / [2][16]; pvw
-// [8][2][MR]; dsm [16][16]; tsm [16]; T [16][17].
+// [8][2][MR]; dsm [16][16]; tsm, ssm (scales) [16]; T [16][17].
 // With VS (V in shared memory) the panel passes through V on its way between
 // global memory and the registers, so that a warp reads and writes 32 consecutive
 // rows of a column there; straight from the registers every access touches 16
 // columns (14 k cycles a panel, with T, at n = 274; 8 k now).
 template <int MR, bool VS>
 __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m, double2* V, double2* T,
-                         double2* red, double2* rowj, double2* pvw, double2* dsm, double2* tsm) {
+                         double2* red, double2* rowj, double2* pvw, double2* dsm, double2* tsm, double2* ssm) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int c = tid & 15, g = tid >> 4;
   const int Mt = m / kNB;  // m is a multiple of 16: row slots t < Mt are inside the panel
@@ -264,7 +265,10 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
     const Refl R = make_refl(alpha, xn);
     // w_c = conj(tau) v^H a_c (v = (1; scal a_j)); a_c -= v w_c
     const double2 w = cmul(cconj(R.tau), cadd(rj, cmulc(R.scal, tot)));
-    const double2 sw = c > j ? cmul(R.scal, w) : (c == j ? make_double2(1.0 - R.scal.x, -R.scal.y) : make_double2(0, 0));
+    const double2 sc = cmul(R.scal, w);
+    const long long up = c > j ? ~0ll : 0ll;  // a mask, so that no branch goes around the products
+    const double2 sw = make_double2(__longlong_as_double(__double_as_longlong(sc.x) & up),
+                                    __longlong_as_double(__double_as_longlong(sc.y) & up));
     if (g > j) cfms(col[0], pv[0], sw);
 #pragma unroll
     for (int t0 = 0; t0 < MR; t0 += 4) {
@@ -279,8 +283,9 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
       }
     }
     if (g == j) col[0] = c > j ? csub(col[0], w) : (c == j ? make_double2(R.beta, 0.0) : col[0]);
-    if (g == 0 && c < j) dsm[j * 16 + c] = cadd(cconj(rj), cmul(R.scal, cconj(tot)));  // v_c^H v_j
-    if (tid == 0) tsm[j] = R.tau;
+    if (g == 2 && c < j) dsm[j * 16 + c] = cadd(cconj(rj), cmul(R.scal, cconj(tot)));  // v_c^H v_j / conj(scal_c)
+    if (tid == 64) tsm[j] = R.tau;
+    if (tid == 96) ssm[j] = R.scal;
     // the next pivot column reaches the group through the warp's buffer
     __syncwarp();
     if (j + 1 < kNB && c == j + 1) {
@@ -291,6 +296,7 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
     __syncwarp();
   }
   __syncthreads();
+  if (c < g) dsm[g * 16 + c] = cmulc(ssm[c], dsm[g * 16 + c]);
   // R and the reflectors back in place (band and back-transform); V explicit
   // (unit diagonal, zeros above it)
   if (VS) {
@@ -299,9 +305,15 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
       if (t < Mt) V[pidx(g + 16 * t, c)] = col[t];
     __syncthreads();
 #pragma unroll 2
-    for (int cc = wid; cc < kNB; cc += kNW)
+    for (int cc = wid; cc < kNB; cc += kNW) {
+      const double2 own = ssm[cc];
 #pragma unroll 4
-      for (int r = lane; r < m; r += 32) Ap[(size_t)cc * ld + r] = V[pidx(r, cc)];
+      for (int r = lane; r < m; r += 32) {
+        const double2 v = V[pidx(r, cc)], x = r > cc ? cmul(v, own) : v;
+        V[pidx(r, cc)] = x;
+        Ap[(size_t)cc * ld + r] = x;
+      }
+    }
     __syncthreads();
     if (g <= c) V[pidx(g, c)] = make_double2(g == c ? 1.0 : 0.0, 0.0);
   } else {
@@ -309,10 +321,12 @@ __device__ void panel_qr(double2* __restrict__ A, int ld, int c0, int r0, int m,
     for (int t = 0; t < MR; ++t) {
       const int r = g + 16 * t;
       if (t < Mt) {
-        Ap[(size_t)c * ld + r] = col[t];
-        V[pidx(r, c)] = r < c ? make_double2(0, 0) : (r == c ? make_double2(1, 0) : col[t]);
+        const double2 v = r > c ? cmul(col[t], ssm[c]) : col[t];
+        Ap[(size_t)c * ld + r] = v;
+        V[pidx(r, c)] = r < c ? make_double2(0, 0) : (r == c ? make_double2(1, 0) : v);
       }
     }
+    __syncthreads();
   }
   // T[0:j, j] = -tau_j T[0:j, 0:j] (v_0 .. v_{j-1})^H v_j (zlarft), column after
   // column: lane i of warp 0 keeps row i, its two halves take every other term
@@ -536,7 +550,7 @@ __global__ void __launch_bounds__(kThr, OCC) sb_kernel(const EigItem* __restrict
 
   for (int c0 = 0; c0 + kNB < ld; c0 += kNB) {
     const int r0 = c0 + kNB, m = ld - r0, Mt = m / kNB;
-    panel_qr<MR, !KVG>(A, ld, c0, r0, m, S.V, S.T, S.part, S.rowj, S.pvw, S.M, S.taus);
+    panel_qr<MR, !KVG>(A, ld, c0, r0, m, S.V, S.T, S.part, S.rowj, S.pvw, S.M, S.taus, S.P);
     // T into the free upper tile (rows c0.., columns r0..) for the back-transform
     for (int idx = tid; idx < kNB * kNB; idx += kThr) {
       const int i = idx % kNB, j = idx / kNB;
