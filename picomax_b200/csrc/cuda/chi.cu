@@ -505,8 +505,8 @@ namespace dev {
 // warps over rows: bound by the latency of
 // the n steps, so that several CTAs share an SM (four of 59 vectors; four warps of
 // one CTA had a matrix each before, with a serial back substitution). Measured on a
-// B200, 2000 frequencies: 59 vectors 2.06 -> 0.58 ms, 27 vectors 0.138 -> 0.089 ms, 15
-// vectors 0.058 -> 0.046 ms.
+// B200, 2000 frequencies: 59 vectors 2.06 -> 0.60 ms, 27 vectors 0.138 -> 0.091 ms, 15
+// vectors 0.058 -> 0.047 ms.
 __global__ void __launch_bounds__(128) epsm_kernel(const double* __restrict__ re, const double* __restrict__ im,
                                                    int neps, int nf, double2* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smraw[];

@@ -194,11 +194,13 @@ __host__ __device__ inline size_t sb_smem_bytes(int ld, int mr, bool yg, bool vg
 // sums in shared memory. The update of the columns has one form for every
 // column, a_c[r] -= a_j[r] s_c (s_c = scal w_c for c > j, else 0), so that the lanes
 // of a warp do not diverge; the columns keep a_c unscaled and become v_c = scal a_c at
-// the end (a_c - a_c (1 - scal) lost eps |A| of v_c, all of it at |A| = 1e16). Rows go four at a
-// time (slots past the panel hold zeros), so that four loads of the pivot column
-// and four chains are in flight: with a check per row the two warps of a scheduler
-// waited for one load after another at large n. The pivot column reaches the threads of a row group through the warp's own shared-memory buffer (the
-// group's 16 threads share a warp). red/rowj: [2][8][16] / [2][16]; pvw
+// the end (a_c - a_c (1 - scal) in the common update lost eps |A| of v_c, all of it at
+// |A| = 1e16; 296 matrices of n = 274 5.17 -> 5.25 ms, 148 of n = 401 7.48 -> 7.43, of
+// n = 570 17.2 -> 17.5). Rows go four at a time (slots past the panel hold zeros), so
+// that four loads of the pivot column and four chains are in flight: with a check per
+// row the two warps of a scheduler waited for one load after another at large n. The
+// pivot column reaches the threads of a row group through the warp's own shared-memory
+// buffer (the group's 16 threads share a warp). red/rowj: [2][8][16] / [2][16]; pvw
 // [8][2][MR]; dsm [16][16]; tsm, ssm (scales) [16]; T [16][17].
 // With VS (V in shared memory) the panel passes through V on its way between
 // global memory and the registers, so that a warp reads and writes 32 consecutive

@@ -454,10 +454,10 @@ DevCrystal upload_crystal(pmx_ctx* c, const pmx_problem* P, int force_spinor) {
 // schedules are offered. A launch's items then carry the padded leading dimension
 // and a slot of the band reflector buffer (ctx rbuf).
 // The line at 96, measured on a B200 (two-stage / one-stage, whose matrix fits in
-// shared memory up to n = 153): n = 96 41 matrices 0.48 / 0.59 ms, 433 1.05 / 1.30, 1025
-// 2.16 / 2.71; n = 113 122 0.71 / 0.85, 433 1.61 / 2.54, 1025 3.31 / 5.90; 1025 of n = 137
-// 4.03 / 9.93; 433 of n = 153 2.39 / 4.99. Below, the padding to 96 takes up to 1.7 times
-// the work: n = 81 41 0.47 / 0.47, 433 1.00 / 1.04, 1025 2.04 / 2.15; n = 88 433 1.02 / 1.15
+// shared memory up to n = 153): n = 96 41 matrices 0.48 / 0.59 ms, 433 1.10 / 1.30, 1025
+// 2.19 / 2.71; n = 113 122 0.70 / 0.85, 433 1.64 / 2.54, 1025 3.34 / 5.90; 1025 of n = 137
+// 4.07 / 9.92; 433 of n = 153 2.40 / 4.98. Below, the padding to 96 takes up to 1.7 times
+// the work: n = 81 41 0.47 / 0.47, 433 1.02 / 1.03, 1025 2.11 / 2.15; n = 88 433 1.08 / 1.15
 // (the line was drawn when both stages still ran one CTA per SM and n = 81 took 1.19 ms).
 constexpr int kTwoStageMin = 96;
 bool use_two_stage(int max_n, bool tri) {
